@@ -9,22 +9,9 @@
 // kernels), so every CTA stays busy until the batch is empty whatever the mix of
 // code sizes and per-word iteration counts.  Shared memory is sized for the
 // largest code of the batch.
-#include "decode_kernel.cuh"
+#include "batch_kernel.cuh"
 
 namespace ldpc {
-
-struct BatchCode {
-    Plan plan;
-    const int8_t* llr;      // frame-major int8, 4 * words frames
-    void* out;              // 0/1 bytes (or packed bits), frame-major
-    int32_t* iters_out;     // [words] or null
-    uint8_t* synd_out;      // [4 * words] per-frame syndrome flags or null
-    long long words;
-    long long first_item;   // items of the codes before this one
-    int quirk;              // OMS first-iteration quirk (row classes of this code)
-    int out_packed;
-    int variant;            // this code's row-degree class: 0 <= 8, 1 <= 16, 2 <= 32
-};
 
 // VMAX: the largest degree class of the batch; each word runs the unrolled update
 // of its own code's class
@@ -41,18 +28,8 @@ __global__ void __launch_bounds__(256) decode_batch_kernel(const BatchCode* __re
         __syncthreads();
         const long long item = s_item;
         if (item >= total) break;  // uniform
-        int c = 0;
-        while (c + 1 < n_codes && item >= codes[c + 1].first_item) c++;
-        const BatchCode& bc = codes[c];
-        Job J = base;
-        J.llr = bc.llr;
-        J.out = bc.out;
-        J.out_packed = bc.out_packed;
-        J.iters_out = bc.iters_out;
-        J.synd_out = bc.synd_out;
-        J.total_words = bc.words;
-        J.word0 = 0;
-        J.quirk = bc.quirk;
+        Job J;
+        const BatchCode& bc = batch_item(codes, n_codes, item, base, J);
         const Plan P = bc.plan;
         const long long g = item - bc.first_item;
         if (VMAX == 0 || bc.variant == 0)
@@ -98,13 +75,14 @@ const void* kernel_table_batch_pf(int kind, int variant)
 size_t batch_code_bytes() { return sizeof(BatchCode); }
 
 // fills one BatchCode record on the host (the struct stays private to this file)
-void batch_code_fill(void* rec, const Plan& plan, const int8_t* llr, void* out, int32_t* iters_out, uint8_t* synd_out,
+void batch_code_fill(void* rec, const Plan& plan, const LevelPlan& lplan, const int8_t* llr, void* out, int32_t* iters_out, uint8_t* synd_out,
                      long long words, long long first_item, int quirk, int out_packed, int variant)
 {
     BatchCode* b = reinterpret_cast<BatchCode*>(rec);
     b->synd_out = synd_out;
     b->variant = variant;
     b->plan = plan;
+    b->lplan = lplan;
     b->llr = llr;
     b->out = out;
     b->iters_out = iters_out;

@@ -1,0 +1,6 @@
+#include "kernels_level.cuh"
+
+namespace ldpc {
+extern const void* const level_kernels_f1_e2[4][3];
+const void* const level_kernels_f1_e2[4][3] = {LDPC_LEVEL_ROWS(1, 2)};
+}  // namespace ldpc

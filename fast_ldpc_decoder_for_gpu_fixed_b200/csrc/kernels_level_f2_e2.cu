@@ -1,0 +1,6 @@
+#include "kernels_level.cuh"
+
+namespace ldpc {
+extern const void* const level_kernels_f2_e2[4][3];
+const void* const level_kernels_f2_e2[4][3] = {LDPC_LEVEL_ROWS(2, 2)};
+}  // namespace ldpc

@@ -19,6 +19,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -27,6 +28,7 @@
 
 #include "../../include/ldpc_b200.h"
 #include "frame_kernel.cuh"
+#include "level_schedule.h"
 #include "qc_kernel.cuh"
 
 using namespace ldpc;
@@ -111,6 +113,10 @@ struct ldpc_decoder {
     // 3 = one frame per CTA, 4 = QC register-message, 2 frames per CTA, 5 = QC register-message with
     // per-frame early stop and lane refill (persistent CTAs)
     int path = 0;
+    // paths 0 and 2 on decode_level_bytes_kernel: its schedule (level_setup)
+    bool bytes = false;
+    LevelPlan lplan{};
+    unsigned char* d_level = nullptr;
     bool pf_levels = false;  // path 0 with the per-frame early stop (SIMD4; counts per frame)
     bool frame2 = false;     // path 3 with two frames per CTA (decode_frame2_kernel)
     int sms = 0;  // paths 3 and 5: multiprocessors (grid size)
@@ -337,6 +343,8 @@ const void* kernel_table_f16x2h(int kind, int variant);
 const void* kernel_table_frame(int kind, int variant, bool et);
 const void* kernel_table_frame2(int kind, int variant, bool et);
 const void* kernel_table_flood(int kind, int variant);
+const void* kernel_table_level(int kind, int nv, int fp, int et);
+const void* kernel_table_level_half(int kind, int nv);
 }
 
 // shared memory of the QC kernel: the APP, 4 bytes per variable per pair of frames
@@ -469,6 +477,7 @@ static void decoder_free(ldpc_decoder* d)
     cudaFree(d->d_edge_orig);
     cudaFree(d->d_vptr);
     cudaFree(d->d_vedge);
+    cudaFree(d->d_level);
     cudaFree(d->d_in);
     cudaFree(d->d_out);
     cudaFree(d->d_aux);
@@ -535,6 +544,33 @@ static int decoder_setup(ldpc_decoder* d, const ldpc_code* c)
     P.edge_orig = d->d_edge_orig;
     P.vptr = d->d_vptr;
     P.vedge = d->d_vedge;
+    return LDPC_OK;
+}
+
+// The byte kernel's schedule of the code on the device (d->lplan); *lc = its choices, *ok = false
+// when the code has none.
+static int level_setup(ldpc_decoder* d, const ldpc_code* c, size_t lds, long long words, int fixed_threads,
+                       bool may_half, LevelSchedule* lc, bool* ok)
+{
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
+    const Rows H{c->n, c->m, c->row_ptr.data(), c->cols.data(), c->row_class.data()};
+    *ok = level_choose(H, lds, words, sms, fixed_threads, may_half, *lc);
+    if (!*ok) return LDPC_OK;
+    // records, steps and edge indices in one allocation and one copy
+    const size_t rb = lc->recs.size() * sizeof(uint4), sb = lc->steps.size() * sizeof(LevelStep),
+                 eb = lc->edges.size() * sizeof(int32_t);
+    std::vector<unsigned char> h(rb + sb + eb);
+    memcpy(h.data(), lc->recs.data(), rb);
+    memcpy(h.data() + rb, lc->steps.data(), sb);
+    memcpy(h.data() + rb + sb, lc->edges.data(), eb);
+    CUDA_TRY(cudaMalloc(&d->d_level, h.size()));
+    CUDA_TRY(cudaMemcpy(d->d_level, h.data(), h.size(), cudaMemcpyHostToDevice));
+    d->lplan.rec = reinterpret_cast<const uint4*>(d->d_level);
+    d->lplan.step = reinterpret_cast<const LevelStep*>(d->d_level + rb);
+    d->lplan.edge = reinterpret_cast<const int32_t*>(d->d_level + rb + sb);
+    d->lplan.nstep = (int)lc->steps.size();
+    d->lplan.msg_bytes = lc->msg_bytes;
     return LDPC_OK;
 }
 
@@ -645,6 +681,35 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
     d->fst.nst = (int)st.size();
     d->fst.slot_sz = slot_max;
     d->fst.status = d->d_status;
+    return LDPC_OK;
+}
+
+// Paths 0 and 2 on decode_level_bytes_kernel where it serves the decoder: sets d->bytes and the
+// launch, or leaves d to the older level kernels (LEARNED with fp16 constants, more than 16384
+// variables, rows that repeat a variable, a state that only just fits in their layout).
+static int level_select(ldpc_decoder* d, const ldpc_code* c, int kind, bool half, bool early, bool per_frame, int pack,
+                        int smem_max)
+{
+    if (!(half && kind != LDPC_LEARNED) && pack != LDPC_PACK_SIMD4) return LDPC_OK;
+    const size_t lds = 4 * (size_t)d->plan.npad + (kind == LDPC_LEARNED ? 512 : 0);
+    LevelSchedule lc;
+    bool ok = false;
+    int rc = level_setup(d, c, lds, (long long)d->nb_words, 0, half, &lc, &ok);
+    if (rc || !ok) return rc;
+    const size_t smem = lds + lc.msg_bytes;
+    if (smem + 512 > (size_t)smem_max) return LDPC_OK;
+    bool uniform = true;
+    for (int r = 0; r < c->m && uniform; r++) uniform = c->row_ptr[r + 1] - c->row_ptr[r] == c->dmax;
+    const int nv = uniform ? c->dmax : 0;
+    const int k = kind == LDPC_XMS ? LDPC_OMS : kind;  // KIND_* values equal LDPC_* values
+    d->kfn = lc.half ? kernel_table_level_half(k, nv) : kernel_table_level(k, nv, lc.fp, per_frame ? 2 : (early ? 1 : 0));
+    d->grid_mult = lc.half ? 2 : 1;
+    d->kfn_alt = per_frame || half || kind == LDPC_2NMS ? nullptr : kernel_table_level(k, nv, lc.fp, early ? 0 : 1);
+    d->pf_levels = per_frame;
+    d->path = half ? 2 : 0;
+    d->bytes = true;
+    d->smem = (int)smem;
+    d->threads = lc.threads;
     return LDPC_OK;
 }
 
@@ -815,6 +880,11 @@ extern "C" int ldpc_decoder_create(ldpc_decoder** out, const ldpc_code* c, int k
         d->path = 6;
         d->smem = (int)smem;
         d->threads = std::min(256, std::max(32, (c->m + 31) / 32 * 32));
+    } else if ((rc = level_select(d, c, kind, half, early, per_frame, pack, smem_max)) || d->bytes) {
+        if (rc) {
+            decoder_free(d);
+            return rc;
+        }
     } else if (half) {
         d->kfn = kernel_table_f16x2h(kind == LDPC_XMS ? LDPC_OMS : (kind == LDPC_LEARNED ? 3 : kind), degree_variant(c));
         d->path = 2;
@@ -902,7 +972,7 @@ extern "C" int ldpc_decoder_set_early_stop(ldpc_decoder* d, int enabled, int sla
     if (!enabled && d->pf_levels)
         return fail(LDPC_ERR_ARG, "the per-frame early stop of this decoder cannot be turned off; create one "
                                   "without LDPC_FLAG_EARLY_STOP_FRAMES");
-    if ((d->path == 1 || d->path == 3 || d->path == 4 || d->path == 7) && (enabled != 0) != d->early)
+    if ((d->path == 1 || d->path == 3 || d->path == 4 || d->path == 7 || d->bytes) && d->kfn_alt && (enabled != 0) != d->early)
         std::swap(d->kfn, d->kfn_alt);
     d->early = enabled != 0;
     d->early_slack = (unsigned)slack;
@@ -1058,6 +1128,11 @@ static int launch(ldpc_decoder* d, const int8_t* llr, void* out, int out_packed,
             if (d->smem > 48 * 1024) CUDA_TRY(ldpc_internal_raise_smem(x, d->smem));
             kfn = x;
         }
+    }
+    if (d->bytes) {
+        void* a[] = {(void*)&d->plan, (void*)&d->lplan, (void*)&J};
+        CUDA_TRY(cudaLaunchKernel(kfn, dim3((unsigned)(words * d->grid_mult)), dim3(d->threads), a, d->smem, st));
+        return LDPC_OK;
     }
     void* args[] = {(d->path == 1 || d->path == 4 || d->path == 7) ? (void*)&d->qcp : (void*)&d->plan, (void*)&J};
     CUDA_TRY(cudaLaunchKernel(kfn, dim3((unsigned)(words * d->grid_mult)), dim3(d->threads), args, d->smem, st));
@@ -1323,8 +1398,9 @@ namespace ldpc {
 const void* kernel_table_batch(int pack, int kind, int variant);
 const void* kernel_table_batch_pf(int kind, int variant);
 size_t batch_code_bytes();
-void batch_code_fill(void* rec, const Plan& plan, const int8_t* llr, void* out, int32_t* iters_out, uint8_t* synd_out,
-                     long long words, long long first_item, int quirk, int out_packed, int variant);
+const void* kernel_table_batch_bytes(int kind, int et);
+void batch_code_fill(void* rec, const Plan& plan, const LevelPlan& lplan, const int8_t* llr, void* out, int32_t* iters_out,
+                     uint8_t* synd_out, long long words, long long first_item, int quirk, int out_packed, int variant);
 }  // namespace ldpc
 
 struct ldpc_batch {
@@ -1347,6 +1423,11 @@ struct ldpc_batch {
     void* h_codes = nullptr;           // pinned staging of the same
     unsigned long long* d_counter = nullptr;
     const void* kfn = nullptr;
+    // decode_batch_bytes_kernel: each code's schedule by CTA width (made on first use, then kept:
+    // a queued launch may still read them), empty where some code has none; null when kfn is
+    // another kernel
+    std::map<int, std::vector<ldpc_decoder*>> levels;
+    const std::vector<ldpc_decoder*>* lv = nullptr;
     int threads = 128, smem = 0, ctas_per_sm = 0, grid = 0, sms = 0;
     uint16_t* d_lut = nullptr;
     int lut_its = 0;
@@ -1373,6 +1454,8 @@ static void batch_free(ldpc_batch* b)
 {
     if (!b) return;
     for (auto* d : b->plans) decoder_free(d);
+    for (auto& v : b->levels)
+        for (auto* d : v.second) decoder_free(d);
     for (auto& v : b->pc_dec)
         for (auto* d : v)
             if (d) decoder_free(d);
@@ -1460,6 +1543,33 @@ static int batch_code_decoder(ldpc_batch* b, int i, int cand, ldpc_decoder** out
     return LDPC_OK;
 }
 
+// The byte kernel's schedules of all codes for a CTA width; an empty list when a code has none.
+static int batch_levels(ldpc_batch* b, int threads, const std::vector<ldpc_decoder*>** out)
+{
+    auto it = b->levels.find(threads);
+    if (it == b->levels.end()) {
+        std::vector<ldpc_decoder*> v;
+        bool ok = true;
+        int rc = LDPC_OK;
+        for (size_t i = 0; i < b->codes.size() && ok && !rc; i++) {
+            v.push_back(new ldpc_decoder());
+            v.back()->device = b->device;
+            LevelSchedule lc;
+            const size_t lds = 4 * (size_t)b->plans[i]->plan.npad;
+            rc = level_setup(v.back(), &b->codes[i], lds, 1ll << 30, threads, false, &lc, &ok);
+            v.back()->smem = (int)(lds + lc.msg_bytes);
+        }
+        if (rc || !ok) {
+            for (auto* d : v) decoder_free(d);
+            v.clear();
+        }
+        if (rc) return rc;
+        it = b->levels.emplace(threads, std::move(v)).first;
+    }
+    *out = &it->second;
+    return LDPC_OK;
+}
+
 // selects the strategy: one persistent kernel with this packing, CTA width and
 // resident CTAs per SM (0 = as many as fit), or (per_code) one launch of each
 // code's own level kernel with this packing
@@ -1486,6 +1596,33 @@ static int batch_configure(ldpc_batch* b, int pack, int threads, int ctas_per_sm
         return LDPC_OK;
     }
     const int k = b->kind == LDPC_LEARNED ? 4 : b->kind;
+    const std::vector<ldpc_decoder*>* lv = nullptr;
+    if (pack == LDPC_PACK_SIMD4) {
+        int rc = batch_levels(b, threads, &lv);
+        if (rc) return rc;
+        size_t smem = 0;
+        for (auto* d : *lv) smem = std::max(smem, (size_t)d->smem + lut);
+        const void* f = kernel_table_batch_bytes(b->kind, b->per_frame ? 2 : (b->early ? 1 : 0));
+        int occ = 0;
+        if (!lv->empty() && smem + 1024 <= (size_t)smem_max) {
+            rc = batch_lut(b, pack);
+            if (rc) return rc;
+            CUDA_TRY(ldpc_internal_raise_smem(f, smem));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, smem));
+        }
+        if (occ >= 1) {
+            b->per_code = false;
+            b->pack = pack;
+            b->kfn = f;
+            b->lv = lv;
+            b->threads = threads;
+            b->smem = (int)smem;
+            b->ctas_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, occ) : occ;
+            b->grid = b->ctas_per_sm * b->sms;
+            b->key.clear();
+            return LDPC_OK;
+        }
+    }
     const void* kfn = b->per_frame ? (pack == LDPC_PACK_SIMD4 ? kernel_table_batch_pf(b->kind, b->variant) : nullptr)
                                    : kernel_table_batch(pack, k, b->variant);
     if (!kfn)
@@ -1503,6 +1640,7 @@ static int batch_configure(ldpc_batch* b, int pack, int threads, int ctas_per_sm
     b->per_code = false;
     b->pack = pack;
     b->kfn = kfn;
+    b->lv = nullptr;
     b->threads = threads;
     b->smem = (int)smem;
     b->ctas_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, occ) : occ;
@@ -1622,6 +1760,10 @@ extern "C" int ldpc_batch_set_early_stop(ldpc_batch* b, int enabled, int slack)
     if (b->early != (enabled != 0)) batch_drop_decoders(b);  // per-code decoders: re-created with the flag
     b->early = enabled != 0;
     b->slack = (unsigned)slack;
+    if (b->lv) {  // the early stop is compiled into the byte kernel
+        int rc = batch_configure(b, b->pack, b->threads, b->ctas_per_sm, false);
+        if (rc) return rc;
+    }
     b->key.clear();
     return LDPC_OK;
 }
@@ -1640,7 +1782,7 @@ extern "C" int ldpc_batch_decode(ldpc_batch* b, const int8_t* const* d_llr, void
         return fail(LDPC_ERR_ARG, "LDPC_BATCH_GRAPH: pass a stream (the legacy default stream cannot be captured)");
     const int n = (int)b->plans.size();
     long long total = 0;
-    std::vector<uintptr_t> recs = {(uintptr_t)out_format};
+    std::vector<uintptr_t> recs = {(uintptr_t)out_format, (uintptr_t)b->lv};
     for (int i = 0; i < n; i++) {
         if (n_words[i] > 0 && (!d_llr[i] || !d_out[i]))
             return fail(LDPC_ERR_ARG, "ldpc_batch_decode: null buffer for code %d", i);
@@ -1665,7 +1807,8 @@ extern "C" int ldpc_batch_decode(ldpc_batch* b, const int8_t* const* d_llr, void
         b->staged = recs;
         long long first = 0;
         for (int i = 0; i < n; i++) {
-            batch_code_fill(static_cast<char*>(b->h_codes) + i * batch_code_bytes(), b->plans[i]->plan, d_llr[i],
+            batch_code_fill(static_cast<char*>(b->h_codes) + i * batch_code_bytes(), b->plans[i]->plan,
+                            b->lv ? (*b->lv)[i]->lplan : LevelPlan{}, d_llr[i],
                             d_out[i], d_iters_out ? d_iters_out[i] : nullptr,
                             d_syndrome_ok ? d_syndrome_ok[i] : nullptr, (long long)n_words[i], first,
                             b->kind == LDPC_OMS, out_format == LDPC_OUT_PACKED, b->cls[i]);

@@ -57,11 +57,14 @@ extern "C" {
 
 /* frame packing of the on-chip decoder state */
 /* LDPC_PACK_AUTO: the QC register kernel when the code is QC and one fits (info path 1);
- * else LDPC_PACK_F16X2 (2 frames per CTA, path 2) for MS / OMS / NMS / xMS without early
+ * else LDPC_PACK_F16X2 (path 2) for MS / OMS / NMS / xMS without early
  * stop; else LDPC_PACK_SIMD4; LDPC_PACK_FRAME when no 4-frame state fits.  Every packing
  * gives the same decisions. */
 #define LDPC_PACK_AUTO (-1)
-#define LDPC_PACK_SIMD4 0 /* 4 frames per 32-bit word, saturating byte lanes      */
+/* 4 frames per 32-bit word, saturating byte lanes.  Codes of at most 16384 variables whose
+ * rows hold no variable twice run the byte-storage level kernel (fp16x2 arithmetic on the
+ * bytes); others, and ldpc_decode_noalloc, per-byte SIMD. */
+#define LDPC_PACK_SIMD4 0
 /* 2 frames per 32-bit word, integer-valued fp16 lanes.  On a QC code (ldpc_code_create_qc)
  * whose shape has no 4-frame register kernel (more than 8 block rows or an irregular
  * row degree, such as 24-column bases), an explicit LDPC_PACK_F16X2 selects the QC
@@ -317,8 +320,9 @@ int ldpc_decoder_set_early_stop(ldpc_decoder* dec, int enabled, int slack);
 
 /* info[0..7] = kind, pack, nb_frames (words), threads per CTA, shared bytes
  * per CTA, CTAs per SM, registers per thread, kernel path (0 = level
- * scheduled, 1 = QC register-message, 2 = level scheduled with 2 frames per
- * CTA: LDPC_PACK_F16X2 for every kind but 2NMS, 3 = one frame per CTA with
+ * scheduled, 1 = QC register-message, 2 = level scheduled, fixed iterations:
+ * LDPC_PACK_F16X2 for every kind but 2NMS (4 frames per CTA in byte storage, 2 where the words
+ * leave multiprocessors idle, and 2 in fp16 for the codes and kinds byte storage does not serve), 3 = one frame per CTA with
  * packed row state: LDPC_PACK_FRAME, 4 = QC register-message with 2 frames per
  * CTA, see LDPC_PACK_F16X2, 5 = QC register-message with per-frame early stop,
  * see LDPC_FLAG_EARLY_STOP_FRAMES, 6 = level kernel with the flooding schedule, see
