@@ -102,6 +102,7 @@ struct ldpc_decoder {
     void* d_aux = nullptr;     // staging of iteration counts and syndrome flags for ldpc_decode_host_ex
     cudaStream_t s_comp = nullptr, s_h2d = nullptr, s_d2h = nullptr;
     int threads = 0, smem = 0, ctas_per_sm = 0, regs = 0;
+    int widest = 0;  // rows of the widest level
     const void* kfn = nullptr;
     const void* kfn_alt = nullptr;  // the same kernel with the other early-stop setting (paths 1, 3 and 4)
     // path 1, LDPC_LEARNED: the general, the offset-only (every scale 1.0) and the OMS kernel
@@ -135,11 +136,12 @@ struct ldpc_decoder {
 };
 
 // Row schedule and CTA width of a decoder, for the training kernels (train.cu).
-int ldpc_internal_plan(const ldpc_decoder* d, Plan* plan, int* threads)
+int ldpc_internal_plan(const ldpc_decoder* d, Plan* plan, int* threads, bool* uniform)
 {
     if (!d || !d->d_cols) return -1;
     *plan = d->plan;
-    *threads = std::min(256, std::max(32, (d->threads + 31) / 32 * 32));
+    *threads = std::min(256, std::max(32, (d->widest + 31) / 32 * 32));
+    *uniform = (long long)d->plan.dmax * d->plan.m == d->e;  // every row has the largest degree
     return 0;
 }
 
@@ -531,6 +533,7 @@ static int decoder_setup(ldpc_decoder* d, const ldpc_code* c)
         CUDA_TRY(cudaMemcpy(d->d_vptr, vptr.data(), vptr.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(d->d_vedge, vedge.data(), vedge.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
+    d->widest = c->widest;
     Plan& P = d->plan;
     P.n = c->n;
     P.npad = (c->n + 15) / 16 * 16;

@@ -33,8 +33,16 @@
 // fixed), for the two saturations and for the floor; c's clamp passes the
 // gradient only where 0 < y < 31.  The forward pass records {min1, min2,
 // i1 | i2 << 8, sign bits} per row and iteration (16 bytes), and for weighted
-// iterations before the last the APP (4 bytes per variable) and S_f(t), in a
+// iterations before the last sigmoid - b of every variable (4 bytes) and S_f(t), in a
 // caller-provided stash.
+//
+// The row updates are unrolled for the code's row degrees, so that a row's values stay in
+// registers: with loops over the degree they went through local memory, and the kernel waited
+// on that (1.44 G warp instructions at 0.44 per cycle).  sigmoid - b comes from the forward
+// pass's exp(-|z|) and is kept, so the backward pass evaluates no exponential.
+// N = 4096 QC code, 2048 frames, 10 iterations, every iteration weighted, forward and backward,
+// B200: 2.97 ms before, 1.15 ms now; its stash (0.67 GB) and sigmoids (0.30 GB), written and
+// read once, take 0.3 ms of that.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -53,7 +61,7 @@ struct TrainArgs {
     float* grad_beta;      // [T][2] accumulated
     float* loss;           // [1] accumulated
     uint4* stash;          // [frames][T][m]
-    float* stash_app;      // [frames][T][n]
+    float* stash_app;      // [frames][T][n]: sigmoid(kappa a) - b
     float* stash_s;        // [frames][T]
     const float* weights;  // [T] loss weight per iteration, or null (last only)
     float* app_out;        // [frames][n] final soft output, or null
@@ -90,9 +98,15 @@ __device__ __forceinline__ float pre_mag(float al, float be, float x, int quanti
     return __fsub_rn(quantized ? floorf(p) : p, be);
 }
 
-// BCE(sigmoid(z), b) = softplus(z) - b z, and its derivative sigmoid(z) - b
-__device__ __forceinline__ float bce(float z, float b) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))) - b * z; }
-__device__ __forceinline__ float bce_grad(float z, float b) { return 1.f / (1.f + expf(-z)) - b; }
+// BCE(sigmoid(z), b) = softplus(z) - b z and, in grad, its derivative sigmoid(z) - b: with
+// e = exp(-|z|), 1 / (1 + e) or e / (1 + e) with the sign of b, without cancellation
+__device__ __forceinline__ float bce(float z, bool b, float& grad)
+{
+    const float e = expf(-fabsf(z));
+    const float g = ((z >= 0.f) == b ? e : 1.f) / (1.f + e);
+    grad = b ? -g : g;
+    return fmaxf(z, 0.f) + log1pf(e) - (b ? z : 0.f);
+}
 
 __device__ __forceinline__ float iter_weight(const TrainArgs& A, int t)
 {
@@ -110,7 +124,37 @@ __device__ __forceinline__ float term_grad(const TrainArgs& A, float w, float S)
     return A.frame_loss ? w * expf(-S) * A.inv_frames : w * A.inv_n * A.inv_frames;
 }
 
-__global__ void __launch_bounds__(256) train_kernel(const Plan P, const TrainArgs A)
+// The frame's loss sum S_f over its variables (one part per thread) from the APP in shared
+// memory, and sigmoid - b into g (null: not wanted; may be a itself).  VEC: four variables at a
+// time (n a multiple of 4, the buffers aligned for it).
+template <bool VEC>
+__device__ __forceinline__ float frame_part(const TrainArgs& A, int n, long long f, float kap, const float* a, float* g)
+{
+    float part = 0.f;
+    if (VEC) {
+        for (int q = threadIdx.x; q < (n >> 2); q += blockDim.x) {
+            const float4 x = reinterpret_cast<const float4*>(a)[q];
+            const uchar4 b = A.bits ? __ldg(reinterpret_cast<const uchar4*>(A.bits + f * n) + q) : make_uchar4(0, 0, 0, 0);
+            float4 d;
+            part += bce(kap * x.x, b.x, d.x);
+            part += bce(kap * x.y, b.y, d.y);
+            part += bce(kap * x.z, b.z, d.z);
+            part += bce(kap * x.w, b.w, d.w);
+            if (g) reinterpret_cast<float4*>(g)[q] = d;
+        }
+    } else {
+        for (int v = threadIdx.x; v < n; v += blockDim.x) {
+            float d;
+            part += bce(kap * a[v], A.bits ? A.bits[f * n + v] != 0 : false, d);
+            if (g) g[v] = d;
+        }
+    }
+    return part;
+}
+
+// DT: the rows' degree (EXACT) or the most of it
+template <int DT, bool EXACT, bool VEC>
+__global__ void __launch_bounds__(256, DT <= 8 ? 3 : 2) train_kernel(const Plan P, const TrainArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* a = reinterpret_cast<float*>(smem_raw);    // APP, then its gradient
@@ -121,47 +165,61 @@ __global__ void __launch_bounds__(256) train_kernel(const Plan P, const TrainArg
     const int T = A.T;
 
     for (int i = threadIdx.x; i < 4 * LDPC_LEARNED_MAX_ITERS; i += blockDim.x) gpar[i] = 0.f;
-    for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] = A.llr[f * P.n + v];
+    if (VEC)
+        for (int q = threadIdx.x; q < (P.n >> 2); q += blockDim.x)
+            reinterpret_cast<float4*>(a)[q] = __ldg(reinterpret_cast<const float4*>(A.llr + f * P.n) + q);
+    else
+        for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] = A.llr[f * P.n + v];
     for (int i = threadIdx.x; i < P.dmax * P.m; i += blockDim.x) msg[i] = 0.f;
     __syncthreads();
 
     const float kap = A.kappa[f];
     float floss = 0.f;  // this frame's loss (thread 0)
-    auto bit = [&](int v) { return A.bits ? (float)A.bits[f * P.n + v] : 0.f; };
 
     // ---------------- forward ----------------
     for (int t = 0; t < T; t++) {
+        const float al0 = A.alpha[2 * t], al1 = A.alpha[2 * t + 1], be0 = A.beta[2 * t], be1 = A.beta[2 * t + 1];
         for (int l = 0; l < P.nlevels; l++) {
             const int2 lv = __ldg(P.levels + l);
             for (int r = lv.x + threadIdx.x; r < lv.x + lv.y; r += blockDim.x) {
-                const int d = __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
-                const float al = A.alpha[2 * t + g], be = A.beta[2 * t + g];
-                float tv[32];
+                const int d = EXACT ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
+                const float al = g ? al1 : al0, be = g ? be1 : be0;
+                float tv[DT];
+                int vo[DT];
+#pragma unroll
+                for (int j = 0; j < DT; j++)
+                    if (EXACT || j < d) vo[j] = __ldg(P.cols + j * P.m + r);
+#pragma unroll
+                for (int j = 0; j < DT; j++)
+                    if (EXACT || j < d) tv[j] = fminf(fmaxf(__fsub_rn(a[vo[j]], msg[j * P.m + r]), -128.f), 127.f);
                 float m1 = 127.f, m2 = 127.f;
                 int i1 = 0, i2 = 1;
                 uint32_t pos = 0;
-                for (int j = 0; j < d; j++) {
-                    const int v = __ldg(P.cols + j * P.m + r);
-                    const float x = fminf(fmaxf(__fsub_rn(a[v], msg[j * P.m + r]), -128.f), 127.f);
-                    tv[j] = x;
-                    const float ax = fminf(fabsf(x), 127.f);
-                    pos |= (x > 0.f ? 1u : 0u) << j;
-                    if (ax < m1) {
-                        m2 = m1; i2 = i1; m1 = ax; i1 = j;
-                    } else if (ax < m2) {
-                        m2 = ax; i2 = j;
+#pragma unroll
+                for (int j = 0; j < DT; j++) {
+                    if (EXACT || j < d) {
+                        const float ax = fminf(fabsf(tv[j]), 127.f);
+                        pos |= (tv[j] > 0.f ? 1u : 0u) << j;
+                        const bool lt1 = ax < m1, lt2 = ax < m2;
+                        i2 = lt1 ? i1 : (lt2 ? j : i2);
+                        i1 = lt1 ? j : i1;
+                        m2 = fminf(m2, fmaxf(m1, ax));
+                        m1 = fminf(m1, ax);
                     }
                 }
-                if (i2 == i1) i2 = (i1 + 1) % d;  // all magnitudes 127: any second edge
+                if (i2 == i1) i2 = i1 + 1 < d ? i1 + 1 : 0;  // all other magnitudes 127: any second edge
                 const uint32_t par = __popc(pos) & 1;
                 const float c1 = fminf(fmaxf(pre_mag(al, be, m2, A.quantized), 0.f), 31.f);
                 const float c2 = fminf(fmaxf(pre_mag(al, be, m1, A.quantized), 0.f), 31.f);
-                for (int j = 0; j < d; j++) {
-                    const int v = __ldg(P.cols + j * P.m + r);
-                    const float c = j == i1 ? c1 : c2;
-                    const float mj = (par ^ ((pos >> j) & 1)) ? c : -c;
-                    msg[j * P.m + r] = mj;
-                    a[v] = fminf(fmaxf(__fadd_rn(tv[j], mj), -128.f), 127.f);
+                const uint32_t neg = par ? pos : ~pos;  // bit j: the message of edge j is negative
+#pragma unroll
+                for (int j = 0; j < DT; j++) {
+                    if (EXACT || j < d) {
+                        const float c = j == i1 ? c1 : c2;
+                        const float mj = ((neg >> j) & 1) ? -c : c;
+                        msg[j * P.m + r] = mj;
+                        a[vo[j]] = fminf(fmaxf(__fadd_rn(tv[j], mj), -128.f), 127.f);
+                    }
                 }
                 if (A.backward)
                     A.stash[((size_t)f * T + t) * P.m + r] =
@@ -169,14 +227,11 @@ __global__ void __launch_bounds__(256) train_kernel(const Plan P, const TrainArg
             }
             __syncthreads();
         }
-        // intermediate loss terms: their APPs and S_f(t) are kept for the backward pass
+        // intermediate loss terms: their gradients' sigmoids and S_f(t) are kept for the backward pass
         const float w = iter_weight(A, t);
         if (t < T - 1 && w != 0.f) {
-            float part = 0.f;
-            for (int v = threadIdx.x; v < P.n; v += blockDim.x) {
-                part += bce(kap * a[v], bit(v));
-                if (A.backward) A.stash_app[((size_t)f * T + t) * P.n + v] = a[v];
-            }
+            const float part =
+                frame_part<VEC>(A, P.n, f, kap, a, A.backward ? A.stash_app + ((size_t)f * T + t) * P.n : nullptr);
             const float S = block_sum(part, scratch);  // also orders the reads of a before iteration t+1
             floss += term_loss(A, w, S);
             if (A.backward && threadIdx.x == 0) A.stash_s[(size_t)f * T + t] = S;
@@ -185,82 +240,98 @@ __global__ void __launch_bounds__(256) train_kernel(const Plan P, const TrainArg
 
     // ---------------- final loss term and its gradient ----------------
     {
-        float part = 0.f;
-        for (int v = threadIdx.x; v < P.n; v += blockDim.x) {
-            if (A.app_out) A.app_out[f * P.n + v] = a[v];
-            part += bce(kap * a[v], bit(v));
-        }
+        if (A.app_out)
+            for (int v = threadIdx.x; v < P.n; v += blockDim.x) A.app_out[f * P.n + v] = a[v];
+        if (A.app_out) __syncthreads();
         const float w = iter_weight(A, T - 1);
-        const float S = block_sum(part, scratch);
+        const float S = block_sum(frame_part<VEC>(A, P.n, f, kap, a, A.backward ? a : nullptr), scratch);
         floss += term_loss(A, w, S);
-        const float coef = term_grad(A, w, S);
-        for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] = coef * kap * bce_grad(kap * a[v], bit(v));
-        for (int i = threadIdx.x; i < P.dmax * P.m; i += blockDim.x) msg[i] = 0.f;
         if (threadIdx.x == 0) atomicAdd(A.loss, floss);
+        if (!A.backward) return;
+        const float coef = term_grad(A, w, S) * kap;
+        for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] *= coef;
+        for (int i = threadIdx.x; i < P.dmax * P.m; i += blockDim.x) msg[i] = 0.f;
         __syncthreads();
     }
-    if (!A.backward) return;
 
     // ---------------- backward ----------------
     for (int t = T - 1; t >= 0; t--) {
-        float ga[2] = {0.f, 0.f}, gb[2] = {0.f, 0.f};
+        float ga0 = 0.f, ga1 = 0.f, gb0 = 0.f, gb1 = 0.f;
         const float w = iter_weight(A, t);
         if (t < T - 1 && w != 0.f) {  // the loss term on the APP after iteration t
             const float* keep = A.stash_app + ((size_t)f * T + t) * P.n;
-            const float coef = term_grad(A, w, A.stash_s[(size_t)f * T + t]);
-            for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] += coef * kap * bce_grad(kap * keep[v], bit(v));
+            const float coef = term_grad(A, w, A.stash_s[(size_t)f * T + t]) * kap;
+            if (VEC) {
+                for (int q = threadIdx.x; q < (P.n >> 2); q += blockDim.x) {
+                    const float4 k = reinterpret_cast<const float4*>(keep)[q];
+                    float4 x = reinterpret_cast<float4*>(a)[q];
+                    x.x += coef * k.x, x.y += coef * k.y, x.z += coef * k.z, x.w += coef * k.w;
+                    reinterpret_cast<float4*>(a)[q] = x;
+                }
+            } else {
+                for (int v = threadIdx.x; v < P.n; v += blockDim.x) a[v] += coef * keep[v];
+            }
             __syncthreads();
         }
+        const float al0 = A.alpha[2 * t], al1 = A.alpha[2 * t + 1], be0 = A.beta[2 * t], be1 = A.beta[2 * t + 1];
         for (int l = P.nlevels - 1; l >= 0; l--) {
             const int2 lv = __ldg(P.levels + l);
             for (int r = lv.x + threadIdx.x; r < lv.x + lv.y; r += blockDim.x) {
-                const int d = __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
-                const float al = A.alpha[2 * t + g], be = A.beta[2 * t + g];
+                const int d = EXACT ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
                 const uint4 st = A.stash[((size_t)f * T + t) * P.m + r];
+                const float al = g ? al1 : al0, be = g ? be1 : be0;
+                int vo[DT];
+#pragma unroll
+                for (int j = 0; j < DT; j++)
+                    if (EXACT || j < d) vo[j] = __ldg(P.cols + j * P.m + r);
                 const float m1 = __uint_as_float(st.x), m2 = __uint_as_float(st.y);
                 const int i1 = st.z & 0xff, i2 = (st.z >> 8) & 0xff;
-                const uint32_t pos = st.w, par = __popc(pos) & 1;
-                float gt[32];
+                const uint32_t pos = st.w, neg = (__popc(pos) & 1) ? pos : ~pos;
+                float gt[DT];
                 float gc1 = 0.f, gc2 = 0.f;
-                for (int j = 0; j < d; j++) {
-                    const int v = __ldg(P.cols + j * P.m + r);
-                    const float gav = a[v];                    // d/d a[v] after this row
-                    const float gm = gav + msg[j * P.m + r];   // d/d m_j: the APP and the next iteration
-                    gt[j] = gav;
-                    const float s = (par ^ ((pos >> j) & 1)) ? gm : -gm;
-                    if (j == i1) gc1 += s; else gc2 += s;
+#pragma unroll
+                for (int j = 0; j < DT; j++) {
+                    if (EXACT || j < d) {
+                        gt[j] = a[vo[j]];                             // d/d a[v] after this row
+                        const float gm = gt[j] + msg[j * P.m + r];    // d/d m_j: the APP and the next iteration
+                        const float s = ((neg >> j) & 1) ? -gm : gm;
+                        gc1 = j == i1 ? s : gc1;
+                        gc2 += j == i1 ? 0.f : s;
+                    }
                 }
                 float gm1 = 0.f, gm2 = 0.f;
                 const float y1 = pre_mag(al, be, m2, A.quantized), y2 = pre_mag(al, be, m1, A.quantized);
+                float da = 0.f, db = 0.f;
                 if (y1 > 0.f && y1 < 31.f) {
-                    ga[g] += m2 * gc1;
-                    gb[g] -= gc1;
+                    da += m2 * gc1;
+                    db -= gc1;
                     gm2 = al * gc1;
                 }
                 if (y2 > 0.f && y2 < 31.f) {
-                    ga[g] += m1 * gc2;
-                    gb[g] -= gc2;
+                    da += m1 * gc2;
+                    db -= gc2;
                     gm1 = al * gc2;
                 }
+                ga0 += g ? 0.f : da, gb0 += g ? 0.f : db;
+                ga1 += g ? da : 0.f, gb1 += g ? db : 0.f;
                 // min1 = |t_i1|, min2 = |t_i2|; d|t|/dt = +1 for t > 0, -1 otherwise
-                gt[i1] += ((pos >> i1) & 1) ? gm1 : -gm1;
-                gt[i2] += ((pos >> i2) & 1) ? gm2 : -gm2;
-                for (int j = 0; j < d; j++) {
-                    const int v = __ldg(P.cols + j * P.m + r);
-                    a[v] = gt[j];                // d/d a[v] before this row
-                    msg[j * P.m + r] = -gt[j];   // d/d (this edge's message of iteration t-1)
+                gm1 = ((pos >> i1) & 1) ? gm1 : -gm1;
+                gm2 = ((pos >> i2) & 1) ? gm2 : -gm2;
+#pragma unroll
+                for (int j = 0; j < DT; j++) {
+                    if (EXACT || j < d) {
+                        const float x = gt[j] + (j == i1 ? gm1 : (j == i2 ? gm2 : 0.f));
+                        a[vo[j]] = x;              // d/d a[v] before this row
+                        msg[j * P.m + r] = -x;     // d/d (this edge's message of iteration t-1)
+                    }
                 }
             }
             __syncthreads();
         }
+        const float x[4] = {warp_sum(ga0), warp_sum(gb0), warp_sum(ga1), warp_sum(gb1)};
+        if ((threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-            const float x = warp_sum(ga[g]), y = warp_sum(gb[g]);
-            if ((threadIdx.x & 31) == 0) {
-                atomicAdd(&gpar[(2 * t + g) * 2 + 0], x);
-                atomicAdd(&gpar[(2 * t + g) * 2 + 1], y);
-            }
-        }
+            for (int i = 0; i < 4; i++) atomicAdd(&gpar[4 * t + i], x[i]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * T; i += blockDim.x) {
@@ -269,12 +340,22 @@ __global__ void __launch_bounds__(256) train_kernel(const Plan P, const TrainArg
     }
 }
 
+template <bool VEC>
+static const void* train_kernel_for(int dmax, bool uniform)
+{
+    if (uniform && dmax == 6) return (const void*)train_kernel<6, true, VEC>;
+    if (uniform && dmax == 7) return (const void*)train_kernel<7, true, VEC>;
+    if (dmax <= 8) return (const void*)train_kernel<8, false, VEC>;
+    if (dmax <= 16) return (const void*)train_kernel<16, false, VEC>;
+    return (const void*)train_kernel<32, false, VEC>;
+}
+
 }  // namespace ldpc
 
 using namespace ldpc;
 
 int ldpc_internal_fail(int code, const char* msg);
-int ldpc_internal_plan(const ldpc_decoder* dec, Plan* plan, int* threads);
+int ldpc_internal_plan(const ldpc_decoder* dec, Plan* plan, int* threads, bool* uniform);
 cudaError_t ldpc_internal_raise_smem(const void* fn, size_t bytes);
 
 static size_t stash_rows(const Plan& P, size_t frames, int iters) { return frames * (size_t)iters * P.m * sizeof(uint4); }
@@ -284,7 +365,8 @@ extern "C" size_t ldpc_train_stash_bytes(const ldpc_decoder* dec, size_t frames,
 {
     Plan P;
     int threads = 0;
-    if (!dec || iters < 1 || ldpc_internal_plan(dec, &P, &threads)) return 0;
+    bool uniform = false;
+    if (!dec || iters < 1 || ldpc_internal_plan(dec, &P, &threads, &uniform)) return 0;
     return stash_rows(P, frames, iters) + stash_apps(P, frames, iters) + frames * (size_t)iters * sizeof(float);
 }
 
@@ -306,7 +388,8 @@ extern "C" int ldpc_train_step(const ldpc_decoder* dec, const float* d_llr, cons
     if (frames < 1 || frames > 0x7fffffffu) return ldpc_internal_fail(LDPC_ERR_SHAPE, "ldpc_train_step: frames");
     Plan P;
     int threads = 0;
-    if (ldpc_internal_plan(dec, &P, &threads))
+    bool uniform = false;
+    if (ldpc_internal_plan(dec, &P, &threads, &uniform))
         return ldpc_internal_fail(LDPC_ERR_ARG, "ldpc_train_step: decoder has no row schedule");
     if (P.dmax > 32 || P.dmax < 2)
         return ldpc_internal_fail(LDPC_ERR_UNSUPPORTED, "ldpc_train_step: row degrees must be in [2, 32]");
@@ -339,10 +422,13 @@ extern "C" int ldpc_train_step(const ldpc_decoder* dec, const float* d_llr, cons
     A.backward = backward ? 1 : 0;
     A.inv_frames = (float)(1.0 / (double)frames);
     A.inv_n = (float)(1.0 / (double)P.n);
-    cudaError_t e = ldpc_internal_raise_smem((const void*)train_kernel, smem);
+    auto aligned = [](const void* p, size_t to) { return ((uintptr_t)p & (to - 1)) == 0; };
+    const bool vec = P.n % 4 == 0 && aligned(d_llr, 16) && aligned(d_bits, 4) && aligned(A.stash_app, 16);
+    const void* fn = vec ? train_kernel_for<true>(P.dmax, uniform) : train_kernel_for<false>(P.dmax, uniform);
+    cudaError_t e = ldpc_internal_raise_smem(fn, smem);
     if (e == cudaSuccess) {
-        train_kernel<<<(unsigned)frames, threads, smem, (cudaStream_t)stream>>>(P, A);
-        e = cudaGetLastError();
+        void* args[] = {(void*)&P, (void*)&A};
+        e = cudaLaunchKernel(fn, dim3((unsigned)frames), dim3(threads), args, smem, (cudaStream_t)stream);
     }
     return e == cudaSuccess ? LDPC_OK : ldpc_internal_fail(LDPC_ERR_CUDA, cudaGetErrorString(e));
 }
