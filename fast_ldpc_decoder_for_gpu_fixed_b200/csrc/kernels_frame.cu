@@ -23,22 +23,18 @@ const void* kernel_table_frame(int kind, int variant, bool et)
     return table[et ? 1 : 0][row][variant];
 }
 
-#define LDPC_FRAME2_ENTRIES(ET, KIND)                                                                  \
-    {(const void*)decode_frame2_kernel<KIND, 6, true, ET>, (const void*)decode_frame2_kernel<KIND, 7, true, ET>, \
-     (const void*)decode_frame2_kernel<KIND, 8, false, ET>,                                            \
-     (const void*)decode_frame2_kernel<KIND, FRAME_MAX_DEGREE, false, ET>},
+#define LDPC_FRAME2_ENTRIES(ET)                                                                              \
+    {(const void*)decode_frame2_kernel<KIND_MS, ET, false>, (const void*)decode_frame2_kernel<KIND_OMS, ET, false>, \
+     (const void*)decode_frame2_kernel<KIND_NMS, ET, false>, (const void*)decode_frame2_kernel<KIND_LEARNED, ET, false>, \
+     (const void*)decode_frame2_kernel<KIND_OMS, ET, true>}
 
-// two frames per CTA: [early stop][kind: MS, OMS, NMS, LEARNED][variant]
-const void* kernel_table_frame2(int kind, int variant, bool et)
+// two frames per CTA: [early stop][kind: MS, OMS, NMS, LEARNED, OMS with its first-iteration quirk]
+const void* kernel_table_frame2(int kind, bool et, bool quirk)
 {
-    static const void* table[2][4][4] = {
-        {LDPC_FRAME2_ENTRIES(false, KIND_MS) LDPC_FRAME2_ENTRIES(false, KIND_OMS) LDPC_FRAME2_ENTRIES(false, KIND_NMS)
-             LDPC_FRAME2_ENTRIES(false, KIND_LEARNED)},
-        {LDPC_FRAME2_ENTRIES(true, KIND_MS) LDPC_FRAME2_ENTRIES(true, KIND_OMS) LDPC_FRAME2_ENTRIES(true, KIND_NMS)
-             LDPC_FRAME2_ENTRIES(true, KIND_LEARNED)}};
-    const int row = kind == KIND_LEARNED ? 3 : kind;
-    if (kind == KIND_2NMS || row < 0 || row > 3 || variant < 0 || variant > 3) return nullptr;
-    return table[et ? 1 : 0][row][variant];
+    static const void* table[2][5] = {LDPC_FRAME2_ENTRIES(false), LDPC_FRAME2_ENTRIES(true)};
+    const int row = kind == KIND_LEARNED ? 3 : (kind == KIND_OMS && quirk ? 4 : kind);
+    if (kind == KIND_2NMS || row < 0 || row > 4) return nullptr;
+    return table[et ? 1 : 0][row];
 }
 
 }  // namespace ldpc

@@ -343,7 +343,7 @@ const void* kernel_table_qc_split(int kind, int dt, int layers, int split, bool 
 const void* kernel_table_simd4_pf(int kind, int variant);
 const void* kernel_table_f16x2h(int kind, int variant);
 const void* kernel_table_frame(int kind, int variant, bool et);
-const void* kernel_table_frame2(int kind, int variant, bool et);
+const void* kernel_table_frame2(int kind, bool et, bool quirk);
 const void* kernel_table_flood(int kind, int variant);
 const void* kernel_table_level(int kind, int nv, int fp, int et);
 const void* kernel_table_level_half(int kind, int nv);
@@ -582,8 +582,7 @@ static int level_setup(ldpc_decoder* d, const ldpc_code* c, size_t lds, long lon
 // on an SM where the frame allows it) and lays out their records and message offsets,
 // 16-byte aligned for the bulk copies (FrameStage in frame_kernel.cuh).  base_smem: the
 // kernel's shared memory before the ring (the APP and the learned tables).
-// two: the layout of decode_frame2_kernel (edge slots of u16 columns, a 64-byte header, one
-// CTA per SM with two frames' APP).
+// two: the layout of decode_frame2_kernel (one CTA per SM with two frames' APP).
 static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_smem, bool two)
 {
     const int T = d->threads - 32;  // rows per stage; the last warp is the producer's
@@ -592,13 +591,15 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
     CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, d->device));
     CUDA_TRY(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, d->device));
     CUDA_TRY(cudaDeviceGetAttribute(&smem_blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
-    // a stage slot holds the header, the row words, the column pairs and the messages of
-    // its rows: at least one row of the largest degree
-    // entries per row: pairs of edges (one frame), or edges (two frames); 4 bytes of columns
-    // per pair entry or 2 per edge entry, 2 bytes of messages per entry either way
-    const int hdr = two ? FRAME2_HEADER : FRAME_STAGE_HEADER, cb = two ? 2 : 4;
-    auto entries = [&](int dg) { return two ? dg : (dg + 1) / 2; };
-    const long long slot_min = hdr + 16 + pad16((long long)cb * entries(c->dmax)) + pad16(2ll * entries(c->dmax));
+    // a stage slot holds the record and the messages of its rows: at least one row of the
+    // largest degree.  One frame: a header, row words, then per pair of edges 4 bytes of
+    // columns and 2 of messages; two frames: a header, 2 bytes of columns and 2 of messages
+    // per edge of the lists, and a byte per row where they differ
+    const int hdr = two ? FRAME2_HEADER : FRAME_STAGE_HEADER;
+    auto degree = [&](int i) { return c->row_ptr[c->order[i] + 1] - c->row_ptr[c->order[i]]; };
+    auto entries = [&](int dg) { return (dg + 1) / 2; };
+    const long long slot_min = two ? hdr + 2 * pad16(2ll * 14) + 16
+                                   : hdr + 16 + pad16(4ll * entries(c->dmax)) + pad16(2ll * entries(c->dmax));
     const long long static_smem = 512;  // the kernel's static shared memory, rounded up
     long long slot_cap = 0;
     for (int ctas = two ? 1 : 2; ctas >= 1 && slot_cap < slot_min; ctas--) {
@@ -612,54 +613,112 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
     std::vector<unsigned char> rec;
     long long moff = 0;
     int slot_max = 0;
+    auto add_stage = [&](long long rec_bytes, long long msg_bytes) {
+        FrameStage s{};
+        s.rec_bytes = (int)rec_bytes;
+        s.msg_bytes = (int)msg_bytes;
+        s.rec_off = (int)rec.size();
+        s.msg_off = (int)moff;
+        rec.resize(rec.size() + rec_bytes, 0);
+        moff += msg_bytes;
+        slot_max = std::max(slot_max, (int)(rec_bytes + msg_bytes));
+        st.push_back(s);
+        return rec.data() + s.rec_off;
+    };
     auto slot_bytes = [&](int rows, int pairs) {
-        return hdr + pad16(4ll * rows) + pad16((long long)cb * pairs) + pad16(2ll * pairs);
+        return hdr + pad16(4ll * rows) + pad16(4ll * pairs) + pad16(2ll * pairs);
     };
     auto emit = [&](int r0, int rows) {
-        // entry slots (pairs, or edges): rows sorted by decreasing degree, so slot p is a
-        // prefix of the rows
+        // pair slots: rows sorted by decreasing degree, so slot p is a prefix of the rows
         int cnt[16] = {0}, poff[16] = {0};
-        for (int i = 0; i < rows; i++) {
-            const int r = c->order[r0 + i], dg = c->row_ptr[r + 1] - c->row_ptr[r];
-            for (int p = 0; p < entries(dg); p++) cnt[p]++;
-        }
+        for (int i = 0; i < rows; i++)
+            for (int p = 0; p < entries(degree(r0 + i)); p++) cnt[p]++;
         int pairs = 0;
         for (int p = 0; p < 16; p++) {
             poff[p] = pairs;
             pairs += cnt[p];
         }
-        FrameStage s{};
-        const long long cols_off = hdr + pad16(4ll * rows);
-        s.rec_bytes = (int)(cols_off + pad16((long long)cb * pairs));
-        s.msg_bytes = (int)pad16(2ll * pairs);
-        s.rec_off = (int)rec.size();
-        s.msg_off = (int)moff;
-        rec.resize(rec.size() + s.rec_bytes, 0);
-        unsigned char* b = rec.data() + s.rec_off;
+        const long long cols_off = hdr + pad16(4ll * rows), rec_bytes = cols_off + pad16(4ll * pairs);
+        unsigned char* b = add_stage(rec_bytes, pad16(2ll * pairs));
         reinterpret_cast<int32_t*>(b)[0] = rows;
-        reinterpret_cast<int32_t*>(b)[1] = s.rec_bytes;
-        for (int p = 0; p < (two ? 16 : 8); p++) reinterpret_cast<uint16_t*>(b + (two ? 32 : 16))[p] = (uint16_t)poff[p];
+        reinterpret_cast<int32_t*>(b)[1] = (int32_t)rec_bytes;
+        for (int p = 0; p < 8; p++) reinterpret_cast<uint16_t*>(b + 16)[p] = (uint16_t)poff[p];
         for (int i = 0; i < rows; i++) {
             const int r = c->order[r0 + i], e0 = c->row_ptr[r], dg = c->row_ptr[r + 1] - e0;
             reinterpret_cast<uint32_t*>(b + hdr)[i] = (uint32_t)dg | (uint32_t)c->row_class[r] << 8;
-            if (two) {
-                for (int j = 0; j < dg; j++) reinterpret_cast<uint16_t*>(b + cols_off)[poff[j] + i] = (uint16_t)c->cols[e0 + j];
-                continue;
-            }
             for (int p = 0; p < (dg + 1) / 2; p++) {
                 const uint32_t lo = (uint32_t)c->cols[e0 + 2 * p];
                 const uint32_t hi = 2 * p + 1 < dg ? (uint32_t)c->cols[e0 + 2 * p + 1] : 0u;  // odd degree: dummy
                 reinterpret_cast<uint32_t*>(b + cols_off)[poff[p] + i] = lo | hi << 16;
             }
         }
-        moff += s.msg_bytes;
-        slot_max = std::max(slot_max, s.rec_bytes + s.msg_bytes);
-        st.push_back(s);
     };
+    // two frames: rows [r0, r0 + rows) as lists of nv columns, `stride` rows apart; mixed: a byte
+    // per row
+    int stride = 8;
+    auto slot_bytes2 = [&](long long nv, int rows) { return hdr + 2 * pad16(2 * nv * rows) + pad16(rows); };
+    auto emit2 = [&](int r0, int rows, int nv, bool mixed) {
+        const int cls0 = c->row_class[c->order[r0]];
+        const long long list = pad16(2ll * nv * stride), rec_bytes = hdr + list + (mixed ? pad16(rows) : 0);
+        unsigned char* b = add_stage(rec_bytes, list);
+        *reinterpret_cast<Frame2Header*>(b) = {rows, (int)rec_bytes, mixed ? (nv == 4 ? 15 : (nv == 8 ? 16 : 17)) : nv | cls0 << 8,
+                                             st.back().msg_off};
+        for (int i = 0; i < rows; i++) {
+            const int r = c->order[r0 + i], e0 = c->row_ptr[r], dg = degree(r0 + i);
+            // entry j of row i: in the 16-, 8-, 4- or 2-byte part of its list (lv::Msg)
+            for (int j = 0; j < nv; j++) {
+                int base = 0, part = 16;
+                while (base + part > 2 * nv || 2 * j >= base + part) {
+                    if (base + part <= 2 * nv) base += part;
+                    else part >>= 1;
+                }
+                *reinterpret_cast<uint16_t*>(b + hdr + (long long)base * stride + (long long)part * i + (2 * j - base)) =
+                    (uint16_t)(j < dg ? c->cols[e0 + j] : 0);
+            }
+            if (mixed) b[hdr + list + i] = (unsigned char)(dg | c->row_class[r] << 7);
+        }
+    };
+    // two frames: the most rows of a stage, so that the longest lists at that stride fit a slot
+    const int nv_most = c->dmax <= 8 ? std::max(4, c->dmax) : 14;
+    int rows_cap = T;
+    while (two && rows_cap > 8 && slot_bytes2(nv_most, (rows_cap + 7) / 8 * 8) > slot_cap) rows_cap--;
+    // two frames: calls f(first row, rows, list length, mixed) for the stages of a level
+    auto level_stages = [&](const int2& lv, auto f) {
+        const int end = lv.x + lv.y;
+        // rows of a level are sorted by decreasing degree
+        auto cls = [&](int i) { return c->row_class[c->order[i]]; };
+        auto group_end = [&](int r0) {
+            int r1 = r0;
+            while (r1 < end && degree(r1) == degree(r0) && cls(r1) == cls(r0)) r1++;
+            return r1;
+        };
+        int groups = 0;
+        for (int r0 = lv.x; r0 < end; r0 = group_end(r0)) groups++;
+        for (int r0 = lv.x; r0 < end;) {
+            const bool mixed = groups > 2;
+            const int g1 = mixed ? end : group_end(r0), nv = mixed ? frame2_mixed(degree(r0)) : degree(r0);
+            for (int parts = (g1 - r0 + rows_cap - 1) / rows_cap; parts > 0; parts--) {  // equal parts
+                const int rows = (g1 - r0 + parts - 1) / parts;
+                f(r0, rows, nv, mixed);
+                r0 += rows;
+            }
+        }
+    };
+    if (two) {
+        for (const int2& lv : c->levels)
+            level_stages(lv, [&](int, int rows, int, bool) { stride = std::max(stride, (rows + 7) / 8 * 8); });
+        if (slot_bytes2(nv_most, stride) > slot_cap)
+            return fail(LDPC_ERR_UNSUPPORTED, "LDPC_PACK_FRAME: no room for the stage ring next to two frames");
+    }
     for (const int2& lv : c->levels) {
+        const int end = lv.x + lv.y;
+        if (two) {
+            level_stages(lv, emit2);
+            continue;
+        }
         int r0 = lv.x, rows = 0, pairs = 0;
-        for (int i = lv.x; i < lv.x + lv.y; i++) {
-            const int r = c->order[i], np = entries(c->row_ptr[r + 1] - c->row_ptr[r]);
+        for (int i = lv.x; i < end; i++) {
+            const int np = entries(degree(i));
             if (rows > 0 && (rows == T || slot_bytes(rows + 1, pairs + np) > slot_cap)) {
                 emit(r0, rows);
                 r0 = i;
@@ -670,9 +729,18 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
         }
         if (rows) emit(r0, rows);
     }
+    if (two && st.size() < (size_t)FRAME2_STAGES)
+        return fail(LDPC_ERR_UNSUPPORTED, "LDPC_PACK_FRAME: too few stages for two frames per CTA");
     if (rec.size() > (size_t)INT32_MAX || moff > INT32_MAX)
         return fail(LDPC_ERR_UNSUPPORTED, "LDPC_PACK_FRAME: stage records too large");
     CUDA_TRY(cudaMalloc(&d->d_fst, st.size() * sizeof(FrameStage)));
+    // behind the records: the messages of a pair's first iteration (two frames per CTA)
+    const size_t rec_bytes = rec.size();
+    if (two) {
+        int most = 0;
+        for (const FrameStage& x : st) most = std::max(most, x.msg_bytes);
+        rec.resize(rec_bytes + most, 128);
+    }
     CUDA_TRY(cudaMalloc(&d->d_frec, rec.size()));
     CUDA_TRY(cudaMalloc(&d->d_status, sizeof(int)));
     CUDA_TRY(cudaMemcpy(d->d_fst, st.data(), st.size() * sizeof(FrameStage), cudaMemcpyHostToDevice));
@@ -680,6 +748,8 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
     CUDA_TRY(cudaMemset(d->d_status, 0, sizeof(int)));
     d->fst.st = d->d_fst;
     d->fst.rec = d->d_frec;
+    d->fst.none = d->d_frec + rec_bytes;
+    d->fst.stride = stride;
     d->fst.slot_bytes = moff;
     d->fst.nst = (int)st.size();
     d->fst.slot_sz = slot_max;
@@ -833,8 +903,8 @@ extern "C" int ldpc_decoder_create(ldpc_decoder** out, const ldpc_code* c, int k
         // frames per CTA where their APP and a stage ring fit (odd-row counts of a frame below
         // 2^16), else one
         d->threads = std::min(FRAME_MAX_THREADS, std::max(32, (c->widest + 31) / 32 * 32)) + 32;
-        d->frame2 = c->m < 65536 &&
-                    frame_stages_setup(d, c, frame_smem + (size_t)npad, true) == LDPC_OK;
+        d->frame2 = c->m < 65536 && frame_stages_setup(d, c, frame_smem + (size_t)npad, true) == LDPC_OK;
+        const bool quirk = kind == LDPC_OMS && std::find(c->row_class.begin(), c->row_class.end(), 1) != c->row_class.end();
         if (!d->frame2) {
             cudaFree(d->d_fst);
             cudaFree(d->d_frec);
@@ -848,8 +918,8 @@ extern "C" int ldpc_decoder_create(ldpc_decoder** out, const ldpc_code* c, int k
                 return rc;
             }
         }
-        d->kfn = (d->frame2 ? kernel_table_frame2 : kernel_table_frame)(k, degree_variant(c), early);
-        d->kfn_alt = (d->frame2 ? kernel_table_frame2 : kernel_table_frame)(k, degree_variant(c), !early);
+        d->kfn = d->frame2 ? kernel_table_frame2(k, early, quirk) : kernel_table_frame(k, degree_variant(c), early);
+        d->kfn_alt = d->frame2 ? kernel_table_frame2(k, !early, quirk) : kernel_table_frame(k, degree_variant(c), !early);
         d->smem = (int)(frame_smem + (d->frame2 ? (size_t)npad : 0) + (size_t)FRAME_RING * d->fst.slot_sz);
         if (d->smem > smem_max) {
             decoder_free(d);

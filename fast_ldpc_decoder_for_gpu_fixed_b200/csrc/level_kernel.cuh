@@ -53,7 +53,7 @@ namespace lv {
 // every other byte permute).
 struct Regs {
     uint32_t c64, c128;
-    __device__ __forceinline__ Regs(const LevelPlan& L) : c64(L.c64), c128(L.c128) {}
+    __device__ __forceinline__ Regs(uint32_t a, uint32_t b) : c64(a), c128(b) {}
 };
 constexpr uint32_t C1152 = 0x64806480u;
 
@@ -123,11 +123,12 @@ __device__ __forceinline__ uint32_t lut2(uint32_t a, const uint16_t* lut)
 
 // The update of one row (or, with SPLIT, of a lane's part of it) for FP frame pairs.  B[p][j] =
 // 1024 + b and M[p][j] = 1152 + m in, the new ones out; odd[p]: the sign bits set in the lanes
-// whose row is odd.  The pairs are written side by side: their chains are independent, and one
+// whose row is odd.  MIXED: only the first d edges are there.  The pairs are written side by side: their chains are independent, and one
 // warp alone would wait on most of its instructions.
-template <int KIND, int NV, int FP, int PER, bool SPLIT>
+template <int KIND, int NV, int FP, int PER, bool SPLIT, bool MIXED = false>
 __device__ __forceinline__ void row_pairs(const Regs& R, uint32_t (&B)[FP][NV], uint32_t (&M)[FP][NV], bool shortrow,
-                                          int lgs, unsigned wmask, bool noclip, const uint16_t* lut, uint32_t (&odd)[FP])
+                                          int lgs, unsigned wmask, bool noclip, const uint16_t* lut, uint32_t (&odd)[FP],
+                                          int d = NV)
 {
     using namespace h2;
     uint32_t ut[FP][NV], mn1[FP], mn2[FP];
@@ -141,7 +142,11 @@ __device__ __forceinline__ void row_pairs(const Regs& R, uint32_t (&B)[FP][NV], 
         }
 #pragma unroll
     for (int p = 0; p < FP; p++) {
-        if (SPLIT && shortrow) ut[p][NV - 1] = C127;  // no such edge: the neutral magnitude and sign
+        // no such edge: the neutral magnitude and sign
+        if (SPLIT && shortrow) ut[p][NV - 1] = C127;
+#pragma unroll
+        for (int j = 0; j < NV; j++)
+            if (MIXED && j >= d) ut[p][j] = C127;
         mn1[p] = NV == 1 ? ut[p][0] : min_xs(ut[p][0], ut[p][NV > 1 ? 1 : 0]);
         mn2[p] = NV == 1 ? C127 : max_xs(ut[p][0], ut[p][NV > 1 ? 1 : 0]);
     }
@@ -376,7 +381,7 @@ __device__ __forceinline__ void decode_word_bytes(const Plan& P, const LevelPlan
         reinterpret_cast<uint4*>(msgs)[i] = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
     __syncthreads();
 
-    const Regs R(L);
+    const Regs R(L.c64, L.c128);
     int executed = 0;
     bool passed = false;
     unsigned live = 0xFu;
