@@ -370,8 +370,8 @@ static const void* qc_kernel_for(const ldpc_code* c, int kind, QCParams& q, int 
         for (int j = 0; j < c->nb; j++)
             if (c->shifts[i * c->nb + j] >= 0) d++;
         if (d == 0 || d > QC_MAX_DEG) return nullptr;
-        for (int k = 1; k < c->z; k++)
-            if (c->row_class[i * c->z + k] != c->row_class[i * c->z]) return nullptr;
+        for (int k = 0; k < c->z; k++)
+            if (c->row_class[i * c->z + k]) return nullptr;  // the QC kernels know one row class
         deg[i] = d;
         if (i > 0 && d != dt) exact = false;
         dt = std::max(dt, d);
@@ -405,7 +405,6 @@ static const void* qc_kernel_for(const ldpc_code* c, int kind, QCParams& q, int 
             d++;
         }
         q.deg[i] = deg[i];
-        q.cls[i] = c->row_class[i * c->z];
     }
     if (wpt_out) *wpt_out = wpt;
     return f;

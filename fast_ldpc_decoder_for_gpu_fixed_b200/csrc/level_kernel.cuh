@@ -57,13 +57,6 @@ struct Regs {
 };
 constexpr uint32_t C1152 = 0x64806480u;
 
-__device__ __forceinline__ uint32_t sub_sat(uint32_t a, uint32_t b)  // clamp(a - b, 0, 1)
-{
-    uint32_t d;
-    asm("sub.rn.sat.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-
 __device__ __forceinline__ uint32_t off(const uint4& r, int j)
 {
     const uint32_t w = j < 2 ? r.x : (j < 4 ? r.y : (j < 6 ? r.z : r.w));
@@ -155,16 +148,17 @@ __device__ __forceinline__ void row_pairs(const Regs& R, uint32_t (&B)[FP][NV], 
 #pragma unroll
         for (int p = 0; p < FP; p++) {
             const uint32_t lo = min_xs(ut[p][j], ut[p][j + 1]), hi = max_xs(ut[p][j], ut[p][j + 1]);
-            const uint32_t m2 = min_xs(max_xs(mn1[p], lo), min_xs(mn2[p], hi));
+            const uint32_t x = max_xs(mn1[p], lo), y = min_xs(mn2[p], hi);
+            // the last one by magnitude alone: the sign of min2 is not used, and the abs is free here
+            mn2[p] = j + 2 >= NV ? hmin(habs(x), habs(y)) : min_xs(x, y);
             mn1[p] = min_xs(mn1[p], lo);
-            mn2[p] = m2;
         }
 #pragma unroll
     for (int p = 0; p < FP; p++) {
         if ((NV & 1) && NV > 1) {
             const uint32_t mx = max_xs(ut[p][NV - 1], mn1[p]);
             mn1[p] = min_xs(mn1[p], ut[p][NV - 1]);
-            mn2[p] = min_xs(mn2[p], mx);
+            mn2[p] = hmin(habs(mn2[p]), habs(mx));
         }
     }
     if (SPLIT)
@@ -172,7 +166,7 @@ __device__ __forceinline__ void row_pairs(const Regs& R, uint32_t (&B)[FP][NV], 
 #pragma unroll
             for (int p = 0; p < FP; p++) {
                 const uint32_t p1 = __shfl_xor_sync(wmask, mn1[p], o), p2 = __shfl_xor_sync(wmask, mn2[p], o);
-                mn2[p] = min_xs(min_xs(mn2[p], p2), max_xs(mn1[p], p1));
+                mn2[p] = hmin(hmin(habs(mn2[p]), habs(p2)), habs(max_xs(mn1[p], p1)));
                 mn1[p] = min_xs(mn1[p], p1);
             }
     uint32_t c1s[FP], dcs[FP];
@@ -185,12 +179,13 @@ __device__ __forceinline__ void row_pairs(const Regs& R, uint32_t (&B)[FP][NV], 
             mn2[p] = min_xs(mn2[p], C127);
         }
         odd[p] = mn1[p] & SIGN;
+        const uint32_t a2 = NV >= 3 ? mn2[p] : habs(mn2[p]);
         uint32_t c1, c2;
         if (KIND == KIND_LEARNED) {
-            c1 = lut2(habs(mn2[p]), lut);
+            c1 = lut2(a2, lut);
             c2 = lut2(habs(mn1[p]), lut);
         } else {
-            mags<KIND>(habs(mn1[p]), habs(mn2[p]), noclip, c1, c2, 0, 0);
+            mags<KIND>(habs(mn1[p]), a2, noclip, c1, c2, 0, 0);
         }
         c1s[p] = c1 | odd[p];
         dcs[p] = sub(c2 | odd[p], c1s[p]);

@@ -198,6 +198,12 @@ __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b)
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
+__device__ __forceinline__ uint32_t sub_sat(uint32_t a, uint32_t b)  // clamp(a - b, 0, 1)
+{
+    uint32_t d;
+    asm("sub.rn.sat.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
 __device__ __forceinline__ uint32_t hmin(uint32_t a, uint32_t b)
 {
     uint32_t d;
@@ -233,7 +239,7 @@ __device__ __forceinline__ uint32_t floor_scale(uint32_t m, uint32_t k, uint32_t
 // row magnitudes from |min1| (a1) and |min2| (a2); lk, lb: the LEARNED (k, k), (b, b) words
 template <int KIND>
 __device__ __forceinline__ void mags(uint32_t a1, uint32_t a2, bool noclip, uint32_t& c1, uint32_t& c2, uint32_t lk,
-                                     uint32_t lb, uint32_t clip = C31)
+                                     uint32_t lb)
 {
     if (KIND == KIND_LEARNED_OFS) {
         // scale 1: clamp(a - offset, 0, 31) with lb = (-offset, -offset), exact on integers
@@ -251,9 +257,9 @@ __device__ __forceinline__ void mags(uint32_t a1, uint32_t a2, bool noclip, uint
     } else if (KIND == KIND_OMS) {
         c1 = fma_relu(a2, ONE, NEG1);
         c2 = fma_relu(a1, ONE, NEG1);
-        if (!noclip) {  // clip: C31, or per lane C31 / no clip (the first iteration of a lane's frame)
-            c1 = hmin(c1, clip);
-            c2 = hmin(c2, clip);
+        if (!noclip) {
+            c1 = hmin(c1, C31);
+            c2 = hmin(c2, C31);
         }
     } else {
         c2 = floor_scale(a1, C075, CNEG0375);
@@ -274,11 +280,11 @@ __device__ __forceinline__ void learned_kb(const uint16_t* lut, uint32_t& lk, ui
 }
 
 // CMODE 0: ov counts odd (row, frame) pairs; 1: ov counts odd rows per fp16 lane (bit 0 and
-// bit 16 fields), and clip is the per-lane OMS clip word; 2: ov is a count_parity
+// bit 16 fields); 2: ov is a count_parity
 // accumulator (+1 per even row, -1 per odd row and lane, on the FMA pipe)
 template <int KIND, int DT, bool EXACT, int CMODE = 0>
 __device__ __forceinline__ void row(uint32_t (&b)[DT], uint32_t (&m)[DT], int d, bool noclip, uint32_t& ov,
-                                    uint32_t lk, uint32_t lb, uint32_t clip = C31)
+                                    uint32_t lk, uint32_t lb)
 {
     uint32_t ut[DT];
     uint32_t mn1 = C127, mn2 = C127;
@@ -298,20 +304,21 @@ __device__ __forceinline__ void row(uint32_t (&b)[DT], uint32_t (&m)[DT], int d,
 #pragma unroll
         for (int j = 2; j + 1 < DT; j += 2) {
             const uint32_t lo = min_xs(ut[j], ut[j + 1]), hi = max_xs(ut[j], ut[j + 1]);
-            const uint32_t m2 = min_xs(max_xs(mn1, lo), min_xs(mn2, hi));
+            const uint32_t x = max_xs(mn1, lo), y = min_xs(mn2, hi);
+            // the last one by magnitude alone: the sign of min2 is not used, and the abs is free here
+            mn2 = j + 2 >= DT ? hmin(habs(x), habs(y)) : min_xs(x, y);
             mn1 = min_xs(mn1, lo);
-            mn2 = m2;
         }
         if (DT & 1) {
             const uint32_t mx = max_xs(ut[DT - 1], mn1);
             mn1 = min_xs(mn1, ut[DT - 1]);
-            mn2 = min_xs(mn2, mx);
+            mn2 = hmin(habs(mn2), habs(mx));
         }
         // The reference starts both minima at 127; |t| reaches 128 only for x = -128.  That
         // changes a magnitude only where the magnitude is not clipped to 31 (NMS, 2NMS,
         // LEARNED, the OMS first-iteration no-clip), so only those cap.
         if (KIND == KIND_NMS || KIND == KIND_2NMS || KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS ||
-            (KIND == KIND_OMS && (noclip || clip != C31))) {
+            (KIND == KIND_OMS && noclip)) {
             mn1 = min_xs(mn1, C127);
             mn2 = min_xs(mn2, C127);
         }
@@ -328,19 +335,19 @@ __device__ __forceinline__ void row(uint32_t (&b)[DT], uint32_t (&m)[DT], int d,
             }
         }
     }
-    const uint32_t a1 = habs(mn1), a2 = habs(mn2);
+    const uint32_t a1 = habs(mn1), a2 = EXACT && DT >= 4 ? mn2 : habs(mn2);
     uint32_t c1, c2;
-    mags<KIND>(a1, a2, noclip, c1, c2, lk, lb, clip);
+    mags<KIND>(a1, a2, noclip, c1, c2, lk, lb);
     const uint32_t c1s = c1 | (mn1 & SIGN), c2s = c2 | (mn1 & SIGN);
-    const uint32_t dcs = sub(c2s, c1s), na1 = a1 ^ SIGN;
+    const uint32_t dcs = sub(c2s, c1s);
 #pragma unroll
     for (int j = 0; j < DT; j++) {
         if (EXACT || j < d) {
             // |t| >= min1 on every edge, so sat(|t| - min1) is 0 on the minimum edge(s)
             // and 1 elsewhere: r = c1s there, c2s elsewhere (one FMA instead of a
             // compare and a select)
-            // (abs.f16x2 rather than a mask: the abs folds into the saturating add)
-            uint32_t r = fma(add_sat(habs(ut[j]), na1), dcs, c1s);
+            // (abs.f16x2 rather than a mask: both fold into the saturating subtract)
+            uint32_t r = fma(sub_sat(habs(ut[j]), habs(mn1)), dcs, c1s);
             uint32_t mo = r ^ (ut[j] & SIGN);                   // flip by this edge's own sign
             m[j] = mo;
             b[j] = hmin(fma_relu(mo, ONE, b[j]), C255);         // clamp(bt + m, 0, 255)

@@ -15,6 +15,12 @@
 // the CTA holds frames 2h, 2h+1 of word g (blockIdx.x = 2 * (g - word0) + h), 4
 // bytes per variable and half the registers, for codes with many layers or
 // high row degrees (24-column bases); its early stop is per frame pair.
+//
+// What bounds it (WPT = 2): the ALU pipe, half rate, with about 7.3 of 14.5 instructions per edge
+// of a frame pair (4.7 min / max, 1.8 logic, 0.5 address), at 75 % busy.  N = 4096, 65 536 frames,
+// 10 iterations, B200: 2.33 ms with the row class looked at in every layer, -|min1| and |min2| made
+// by masks and a no-clip branch that no QC code takes (all its rows are of class 0); 2.14 ms
+// without.  The deployed decoder (early stop per frame pair): 1.57 and 1.54 ms.
 #pragma once
 #include "decode_kernel.cuh"
 
@@ -30,7 +36,7 @@ struct QCParams {
     int layers;
     int zb;                  // bytes of one block column of the APP = vb * z (vb = 4 * WPT bytes per variable)
     int deg[QC_MAX_LAYERS];  // row degree of each layer
-    int cls[QC_MAX_LAYERS];  // reference degree group of each layer (OMS quirk)
+    // (a QC code has one row class, 0: no row of the OMS first-iteration quirk)
     // per (layer, edge): byte offset of the block column in the APP array and the shift
     int cz4[QC_MAX_LAYERS * QC_MAX_DEG];  // vb * c * z
     int s[QC_MAX_LAYERS * QC_MAX_DEG];    // vb * shift
@@ -198,7 +204,6 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
 #pragma unroll
         for (int l = 0; l < L; l++) {
             const int d = EXACT ? DT : Q.deg[l];
-            const bool noclip = J.quirk && it == 0 && Q.cls[l];
             // recompute the 2-instruction addresses each layer instead of pinning
             // L*D of them in registers across iterations (a shared-memory table of
             // them measured slower: the dependent load costs more than it saves)
@@ -221,14 +226,14 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
             }
             uint32_t lk = 0, lb = 0;  // LEARNED constants of this layer's class (registers only within the layer)
             if (KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS) {
-                const uint2 kb = s_kb[lt][Q.cls[l]];
+                const uint2 kb = s_kb[lt][0];
                 lk = kb.x;
                 lb = kb.y;
             }
             // a stopped pair's words are stored back unchanged
-            if (!PAIRS || (live & 1u)) h2::row<KIND, DT, EXACT, CM>(b0, msg[0][l], d, noclip, ov, lk, lb);
+            if (!PAIRS || (live & 1u)) h2::row<KIND, DT, EXACT, CM>(b0, msg[0][l], d, false, ov, lk, lb);
             if (WPT == 2 && (!PAIRS || (live & 2u)))
-                h2::row<KIND, DT, EXACT, CM>(b1, msg[WPT - 1][l], d, noclip, PAIRS ? ov1 : ov, lk, lb);
+                h2::row<KIND, DT, EXACT, CM>(b1, msg[WPT - 1][l], d, false, PAIRS ? ov1 : ov, lk, lb);
 #pragma unroll
             for (int j = 0; j < DT; j++) {
                 if (EXACT || j < d) {
@@ -411,7 +416,6 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
         for (int l = 0; l < L; l++) {
             const int d = Q.deg[l];
             const int nv = d > s ? (d - s + SPLIT - 1) / SPLIT : 0;  // this lane's edges of the row
-            const bool noclip = J.quirk && it == 0 && Q.cls[l];
             int kk = 4 * k;
             asm volatile("" : "+r"(kk));
             int off[DL];
@@ -425,11 +429,11 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][Q.cls[l]];
+                const uint2 kb = s_kb[lt][0];
                 lk = kb.x;
                 lb = kb.y;
             }
-            h2::row_split<KIND, DL, SPLIT, CM>(b, msg[l], nv, noclip, ov, lk, lb, wmask, lead);
+            h2::row_split<KIND, DL, SPLIT, CM>(b, msg[l], nv, false, ov, lk, lb, wmask, lead);
 #pragma unroll
             for (int i = 0; i < DL; i++)
                 if (i < nv) *reinterpret_cast<uint32_t*>(appb + off[i]) = b[i];
@@ -460,8 +464,8 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
 // The 4 frames of a CTA (the fp16 halves of its two pair-words, "lanes" 0..3) are
 // independent: nothing in the row update mixes lanes.  So each lane can run its own
 // frame on its own schedule: the odd-row count, the syndrome check and the iteration
-// limit are evaluated per lane, the learned constants and the OMS first-iteration
-// clip follow each lane's own iteration number, and when a lane's frame stops the
+// limit are evaluated per lane, the learned constants
+// follow each lane's own iteration number, and when a lane's frame stops the
 // CTA writes that frame's decisions and iteration count, puts its next frame into the
 // lane and zeroes the lane's messages.  CTAs are persistent: CTA c of G decodes
 // frames c, c + G, c + 2G, ... (static, so no atomics; at tens of frames per CTA the
@@ -599,7 +603,6 @@ __device__ __forceinline__ void qc_one_pair(const QCParams& Q, const Job& J, cha
 #pragma unroll
         for (int l = 0; l < L; l++) {
             const int d = EXACT ? DT : Q.deg[l];
-            const bool noclip = J.quirk && it == 0 && Q.cls[l];
             int kk = 8 * k;
             asm volatile("" : "+r"(kk));
             int off[DT];
@@ -613,11 +616,11 @@ __device__ __forceinline__ void qc_one_pair(const QCParams& Q, const Job& J, cha
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][Q.cls[l]];
+                const uint2 kb = s_kb[lt][0];
                 lk = kb.x;
                 lb = kb.y;
             }
-            h2::row<KIND, DT, EXACT, 0>(b0, m[l], d, noclip, ov, lk, lb);
+            h2::row<KIND, DT, EXACT, 0>(b0, m[l], d, false, ov, lk, lb);
 #pragma unroll
             for (int j = 0; j < DT; j++)
                 if (EXACT || j < d) *reinterpret_cast<uint32_t*>(appb + off[j]) = b0[j];
@@ -705,7 +708,6 @@ __global__ void __launch_bounds__(256, 2) decode_qc_pairs_kernel(const __grid_co
 #pragma unroll
         for (int l = 0; l < L; l++) {
             const int d = EXACT ? DT : Q.deg[l];
-            const bool noclip = J.quirk && it == 0 && Q.cls[l];
             int kk = 8 * k;
             asm volatile("" : "+r"(kk));
             int off[DT];
@@ -721,12 +723,12 @@ __global__ void __launch_bounds__(256, 2) decode_qc_pairs_kernel(const __grid_co
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][Q.cls[l]];
+                const uint2 kb = s_kb[lt][0];
                 lk = kb.x;
                 lb = kb.y;
             }
-            h2::row<KIND, DT, EXACT, 0>(b0, msg[0][l], d, noclip, ov, lk, lb);
-            h2::row<KIND, DT, EXACT, 0>(b1, msg[1][l], d, noclip, ov, lk, lb);
+            h2::row<KIND, DT, EXACT, 0>(b0, msg[0][l], d, false, ov, lk, lb);
+            h2::row<KIND, DT, EXACT, 0>(b1, msg[1][l], d, false, ov, lk, lb);
 #pragma unroll
             for (int j = 0; j < DT; j++)
                 if (EXACT || j < d) *reinterpret_cast<uint2*>(appb + off[j]) = make_uint2(b0[j], b1[j]);
@@ -818,7 +820,6 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
     __shared__ int s_src[4];           // refill: the slot each done lane takes
     __shared__ int s_head;             // the slot holding the earliest staged frame
     __shared__ __align__(16) uint32_t s_kb[2][4];  // LEARNED, per row group: k words of pair-words 0, 1, then b words
-    __shared__ uint32_t s_clip[2];     // OMS: clip words of second-group rows (per lane: 31, or none in iteration 0)
     __shared__ uint16_t s_tab[QC_LUT_ITS][2][2];  // LEARNED: fp16 (k, b) per iteration and row group
 
     if (k < 2) {
@@ -882,8 +883,6 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
                     h[8 * g + 4 + k] = s_tab[t][g][1];
                 }
             }
-            if (KIND == KIND_OMS)
-                reinterpret_cast<uint16_t*>(s_clip)[k] = (J.quirk && it == 0) ? 0x7bffu : 0x4fc0u;
         }
         __syncthreads();
 
@@ -906,19 +905,14 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
             }
             uint32_t lk0 = 0, lk1 = 0, lb0 = 0, lb1 = 0;
             if (KIND == KIND_LEARNED) {
-                const uint4 q = reinterpret_cast<const uint4*>(s_kb)[Q.cls[l]];
+                const uint4 q = reinterpret_cast<const uint4*>(s_kb)[0];
                 lk0 = q.x;
                 lk1 = q.y;
                 lb0 = q.z;
                 lb1 = q.w;
             }
-            uint32_t cl0 = h2::C31, cl1 = h2::C31;
-            if (KIND == KIND_OMS && Q.cls[l]) {
-                cl0 = s_clip[0];
-                cl1 = s_clip[1];
-            }
-            h2::row<KIND, DT, EXACT, 1>(b0, msg[0][l], d, false, ov0, lk0, lb0, cl0);
-            h2::row<KIND, DT, EXACT, 1>(b1, msg[1][l], d, false, ov1, lk1, lb1, cl1);
+            h2::row<KIND, DT, EXACT, 1>(b0, msg[0][l], d, false, ov0, lk0, lb0);
+            h2::row<KIND, DT, EXACT, 1>(b1, msg[1][l], d, false, ov1, lk1, lb1);
 #pragma unroll
             for (int j = 0; j < DT; j++)
                 if (EXACT || j < d) *reinterpret_cast<uint2*>(appb + off[j]) = make_uint2(b0[j], b1[j]);
