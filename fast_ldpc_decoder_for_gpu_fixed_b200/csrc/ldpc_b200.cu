@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -28,6 +29,7 @@
 
 #include "../../include/ldpc_b200.h"
 #include "frame_kernel.cuh"
+#include "host_pipe.h"
 #include "level_schedule.h"
 #include "qc_kernel.cuh"
 
@@ -99,6 +101,7 @@ struct ldpc_decoder {
     int32_t* d_vedge = nullptr;
     int8_t* d_in = nullptr;    // staging for decode_host (reference: d_MSG_C_2_V as input staging)
     uint8_t* d_out = nullptr;  // staging for decode_host (reference: d_MSG_C_2_V as output staging)
+    bool counted = false;      // known to HostPipes
     void* d_aux = nullptr;     // staging of iteration counts and syndrome flags for ldpc_decode_host_ex
     cudaStream_t s_comp = nullptr, s_h2d = nullptr, s_d2h = nullptr;
     int threads = 0, smem = 0, ctas_per_sm = 0, regs = 0;
@@ -471,6 +474,7 @@ static size_t smem_bytes(int pack, int npad, int dmax, int m)
 static void decoder_free(ldpc_decoder* d)
 {
     if (!d) return;
+    if (d->counted) HostPipes::user(-1);
     cudaFree(d->d_cols);
     cudaFree(d->d_rowdeg);
     cudaFree(d->d_rowcls);
@@ -1272,6 +1276,124 @@ extern "C" int ldpc_simulate(ldpc_decoder* d, size_t n_words, int iters, float s
                   (cudaStream_t)stream, &J);
 }
 
+static int host_decode_status(ldpc_decoder* d)
+{
+    int status = 0;
+    int rc = ldpc_decoder_status(d, &status);
+    if (rc) return rc;
+    if (status) return fail(LDPC_ERR_CUDA, "decode_host: a wait on the copy engine gave up (results invalid)");
+    return LDPC_OK;
+}
+
+// Whether the staged host decode takes the call: both buffers pageable, at least a megabyte of
+// LLRs in the frame-major layout (xMS reads all of its interleaved input at once), a frame's packed
+// decisions within a piece.
+static bool host_pipe_serves(const ldpc_decoder* d, const void* in, const void* out, size_t in_bytes)
+{
+    if (d->kind == LDPC_XMS || in_bytes < (1 << 20) || ((size_t)d->n + 7) / 8 > HostPipe::OUT_BYTES) return false;
+    for (const void* p : {in, out}) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
+
+// Host-buffer decode of all nb_words words between pageable buffers (host_pipe.h): pieces of LLRs
+// through pinned memory, chunks of words decoded as they are complete (on three streams in turn
+// where a decoder's launches may overlap: path 3 shares its message scratch), packed decisions
+// back in pieces of frames, expanded or copied by the team.  *done = false: not available here
+// (memory for the staging), nothing was done.
+static int decode_host_staged(ldpc_decoder* d, const int8_t* llr, uint8_t* out, int iters, int out_format, int32_t* d_its,
+                              uint8_t* d_syn, bool* done)
+{
+    if (!d->counted) {
+        d->counted = true;
+        HostPipes::user(1);
+    }
+    HostPipe* pipe = HostPipes::take(d->device);
+    if (!pipe) return LDPC_OK;
+    HostPipe& P = *pipe;
+    const size_t W = d->nb_words, n = d->n, fb = 4 * n, pb = (n + 7) / 8;
+    const size_t ipw = (d->path == 3 || d->path == 5 || d->pf_levels) ? 4 : 1;
+    const size_t chunks = std::min<size_t>(8, std::max<size_t>(1, W / 128)), per = (W + chunks - 1) / chunks;
+    const size_t frames_piece = std::max<size_t>(1, HostPipe::OUT_BYTES / pb);
+    cudaStream_t comp[3] = {d->s_comp, P.comp[0], P.comp[1]};
+    const int ncomp = d->path == 3 || d->path == 5 ? 1 : 3;
+    struct Piece {
+        size_t f0, frames;
+        int slot;
+    };
+    Piece queue[HostPipe::OUT];
+    int head = 0, queued = 0, in_used = 0, out_used = 0;
+    *done = true;
+    P.team.wake();
+    auto drain = [&]() -> cudaError_t {  // the oldest piece of decisions into the caller's buffer
+        const Piece q = queue[head];
+        head = (head + 1) % HostPipe::OUT;
+        queued--;
+        cudaError_t e = cudaEventSynchronize(P.out_ev[q.slot]);
+        if (e != cudaSuccess) return e;
+        const uint8_t* src = P.out(q.slot);
+        P.team.each([&](int part, int parts) {
+            const size_t a = q.frames * part / parts, b = q.frames * (part + 1) / parts;
+            if (out_format == LDPC_OUT_PACKED)
+                memcpy(out + (q.f0 + a) * pb, src + a * pb, (b - a) * pb);
+            else
+                expand_bits(src + a * pb, out + (q.f0 + a) * n, (int)n, 0, b - a);
+        });
+        return cudaSuccess;
+    };
+    auto run = [&]() -> int {
+        for (size_t c0 = 0, i = 0; c0 < W; c0 += per, i++) {
+            const size_t words = std::min(per, W - c0), bytes = words * fb;
+            cudaStream_t st = comp[i % ncomp];
+            for (size_t o = 0; o < bytes; o += HostPipe::IN_BYTES) {
+                const size_t len = std::min(HostPipe::IN_BYTES, bytes - o);
+                const int s = in_used % HostPipe::IN;
+                if (in_used++ >= HostPipe::IN) CUDA_TRY(cudaEventSynchronize(P.in_ev[s]));
+                const char* src = reinterpret_cast<const char*>(llr) + c0 * fb + o;
+                P.team.each([&](int part, int parts) {
+                    const size_t a = len * part / parts / 64 * 64, b = part + 1 == parts ? len : len * (part + 1) / parts / 64 * 64;
+                    memcpy(P.in(s) + a, src + a, b - a);
+                });
+                CUDA_TRY(cudaMemcpyAsync(d->d_in + c0 * fb + o, P.in(s), len, cudaMemcpyHostToDevice, d->s_h2d));
+                CUDA_TRY(cudaEventRecord(P.in_ev[s], d->s_h2d));
+                while (queued && cudaEventQuery(P.out_ev[queue[head].slot]) == cudaSuccess) CUDA_TRY(drain());
+            }
+            CUDA_TRY(cudaEventRecord(P.chunk_ev, d->s_h2d));
+            CUDA_TRY(cudaStreamWaitEvent(st, P.chunk_ev, 0));
+            const int rc = launch(d, d->d_in + c0 * fb, d->d_out + c0 * 4 * pb, 1, (long long)c0, (long long)words, (long long)W,
+                                  iters, d_its ? d_its + c0 * ipw : nullptr, nullptr, nullptr, st, nullptr,
+                                  d_syn ? d_syn + 4 * c0 : nullptr);
+            if (rc) return rc;
+            CUDA_TRY(cudaEventRecord(P.dec_ev, st));
+            CUDA_TRY(cudaStreamWaitEvent(d->s_d2h, P.dec_ev, 0));
+            for (size_t f = 0; f < 4 * words; f += frames_piece) {
+                if (queued == HostPipe::OUT) CUDA_TRY(drain());
+                const Piece q{4 * c0 + f, std::min(frames_piece, 4 * words - f), out_used++ % HostPipe::OUT};
+                CUDA_TRY(cudaMemcpyAsync(P.out(q.slot), d->d_out + q.f0 * pb, q.frames * pb, cudaMemcpyDeviceToHost, d->s_d2h));
+                CUDA_TRY(cudaEventRecord(P.out_ev[q.slot], d->s_d2h));
+                queue[(head + queued++) % HostPipe::OUT] = q;
+            }
+        }
+        while (queued) CUDA_TRY(drain());
+        return LDPC_OK;
+    };
+    const int rc = run();
+    P.team.rest();
+    if (rc) {
+        cudaDeviceSynchronize();  // no copy into the ring is left behind
+        delete pipe;
+    } else {
+        HostPipes::give(pipe);
+    }
+    return rc;
+}
+
 // Host-buffer decode of all nb_words words: the H2D copy of chunk i+1 and the D2H copy of
 // chunk i-1 overlap the decoding of chunk i (three streams).  out_format selects 0/1 bytes
 // (the reference's) or packed bits; iters_out / synd_out (host, nullable) receive the
@@ -1294,6 +1416,16 @@ static int decode_host_impl(ldpc_decoder* d, const int8_t* llr, void* out, int i
     if ((iters_out || synd_out) && !d->d_aux) CUDA_TRY(cudaMalloc(&d->d_aux, W * 4 * (sizeof(int32_t) + 1)));
     int32_t* d_its = iters_out ? reinterpret_cast<int32_t*>(d->d_aux) : nullptr;
     uint8_t* d_syn = synd_out ? reinterpret_cast<uint8_t*>(d->d_aux) + W * 4 * sizeof(int32_t) : nullptr;
+    if (host_pipe_serves(d, llr, out, W * fb)) {
+        bool done = false;
+        rc = decode_host_staged(d, llr, static_cast<uint8_t*>(out), iters, out_format, d_its, d_syn, &done);
+        if (rc) return rc;
+        if (done) {
+            if (d_its) CUDA_TRY(cudaMemcpy(iters_out, d_its, W * ipw * sizeof(int32_t), cudaMemcpyDeviceToHost));
+            if (d_syn) CUDA_TRY(cudaMemcpy(synd_out, d_syn, W * 4, cudaMemcpyDeviceToHost));
+            return host_decode_status(d);
+        }
+    }
     // chunks of words: copy-in of chunk i+1 and copy-out of chunk i-1 overlap decoding of chunk i
     size_t chunks = (d->kind == LDPC_XMS) ? 1 : std::min<size_t>(8, std::max<size_t>(1, W / 256));
     size_t per = (W + chunks - 1) / chunks;
@@ -1332,11 +1464,7 @@ static int decode_host_impl(ldpc_decoder* d, const int8_t* llr, void* out, int i
     for (auto ev : ev_in) cudaEventDestroy(ev);
     for (auto ev : ev_dec) cudaEventDestroy(ev);
     if (e != cudaSuccess) return fail(LDPC_ERR_CUDA, "decode_host: %s", cudaGetErrorString(e));
-    int status = 0;
-    rc = ldpc_decoder_status(d, &status);
-    if (rc) return rc;
-    if (status) return fail(LDPC_ERR_CUDA, "decode_host: a wait on the copy engine gave up (results invalid)");
-    return LDPC_OK;
+    return host_decode_status(d);
 }
 
 extern "C" int ldpc_decoder_status(ldpc_decoder* d, int* status)
