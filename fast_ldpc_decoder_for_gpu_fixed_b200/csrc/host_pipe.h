@@ -16,14 +16,15 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 namespace ldpc {
 
@@ -34,9 +35,10 @@ public:
     explicit HostTeam(int helpers)
     {
         try {
+            threads_.reserve(helpers);
             for (int i = 0; i < helpers; i++) threads_.emplace_back([this, i] { run(i + 1); });
-        } catch (const std::system_error&) {
-            // no more threads here: the caller and those that started do the work
+        } catch (const std::exception&) {
+            // no more threads or memory here: the caller and those that started do the work
         }
     }
     ~HostTeam()
@@ -201,9 +203,13 @@ public:
         }
         delete p;
     }
-    // a decoder came (+1) or went (-1); the idle pipes go with the last one
+    // a decoder came (+1) or went (-1); the idle pipes go with the last one.  A forked child has
+    // copies of the pipes without their threads: a decoder that it frees leaves them alone, as
+    // joining those threads would wait for good.
     static void user(int change)
     {
+        static const pid_t owner = getpid();
+        if (getpid() != owner) return;
         std::vector<HostPipe*> gone;
         {
             std::lock_guard<std::mutex> l(lock());
