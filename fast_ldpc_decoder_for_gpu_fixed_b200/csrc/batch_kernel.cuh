@@ -18,13 +18,17 @@ struct BatchCode {
     int variant;            // this code's row-degree class: 0 <= 8, 1 <= 16, 2 <= 32
 };
 
-// The job of item `item` of the batch: its code's record, the word in that code.
-__device__ __forceinline__ const BatchCode& batch_item(const BatchCode* codes, int n_codes, long long item, const Job& base,
-                                                       Job& J)
+// The code of item `item` of the batch.
+__device__ __forceinline__ int batch_code_of(const BatchCode* codes, int n_codes, long long item)
 {
     int c = 0;
     while (c + 1 < n_codes && item >= codes[c + 1].first_item) c++;
-    const BatchCode& bc = codes[c];
+    return c;
+}
+
+// J = the batch's job with the buffers of code bc.
+__device__ __forceinline__ void batch_job(const BatchCode& bc, const Job& base, Job& J)
+{
     J = base;
     J.llr = bc.llr;
     J.out = bc.out;
@@ -34,6 +38,14 @@ __device__ __forceinline__ const BatchCode& batch_item(const BatchCode* codes, i
     J.total_words = bc.words;
     J.word0 = 0;
     J.quirk = bc.quirk;
+}
+
+// The job of item `item` of the batch: its code's record, the word in that code.
+__device__ __forceinline__ const BatchCode& batch_item(const BatchCode* codes, int n_codes, long long item, const Job& base,
+                                                       Job& J)
+{
+    const BatchCode& bc = codes[batch_code_of(codes, n_codes, item)];
+    batch_job(bc, base, J);
     return bc;
 }
 
