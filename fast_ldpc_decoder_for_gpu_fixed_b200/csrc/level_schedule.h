@@ -228,10 +228,17 @@ inline bool level_choose(const Rows& H, size_t lds, long long words, int sms, in
     const int regs = uniform && (H.degree(0) == 6 || H.degree(0) == 7) ? 72 : 96;
     double best_cost = 0;
     size_t last_steps = 0;
-    for (int most : {32, 64, 96, 128, 256}) {
+    const int widths[] = {32, 64, 96, 128, 256};
+    // the widest that the CTA allows is always considered, so that a wide code has a schedule at any
+    // width of the batch's persistent kernel (short irregular codes and a Z = 256 code, 12 500 words,
+    // early stop, 128 threads: 1.86 ms; 7.70 ms on the per-byte kernel that serves a batch without one)
+    int widest_most = 256;
+    for (int most : widths)
+        if (!fixed_threads || most <= fixed_threads) widest_most = most;
+    for (int most : widths) {
+        if (most > widest_most) break;
         // too narrow for the code: many more steps than its longest chain
-        if (most < 256 && (long long)most * order.least() * 3 < 2ll * H.m) continue;
-        if (fixed_threads && most > fixed_threads) break;
+        if (most < widest_most && (long long)most * order.least() * 3 < 2ll * H.m) continue;
         order.steps(most, cur);
         if (last_steps == cur.end.size()) break;  // no step is wider than before
         last_steps = cur.end.size();
