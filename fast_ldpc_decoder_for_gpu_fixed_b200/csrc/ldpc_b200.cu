@@ -1629,6 +1629,7 @@ struct ldpc_batch {
     std::map<int, std::vector<ldpc_decoder*>> levels;
     const std::vector<ldpc_decoder*>* lv = nullptr;
     int threads = 128, smem = 0, ctas_per_sm = 0, grid = 0, sms = 0;
+    int ctas_asked = 0;  // resident CTAs per SM that were asked for (0 = as many as fit)
     uint16_t* d_lut = nullptr;
     int lut_its = 0;
     std::vector<int8_t> off;
@@ -1770,6 +1771,16 @@ static int batch_levels(ldpc_batch* b, int threads, const std::vector<ldpc_decod
     return LDPC_OK;
 }
 
+// the per-code strategy with the per-code choices as they stand
+static void batch_use_per_code(ldpc_batch* b)
+{
+    b->per_code = true;
+    b->kfn = nullptr;
+    b->lv = nullptr;
+    b->grid = b->threads = b->smem = b->ctas_per_sm = 0;
+    b->key.clear();
+}
+
 // selects the strategy: one persistent kernel with this packing, CTA width and
 // resident CTAs per SM (0 = as many as fit), or (per_code) one launch of each
 // code's own level kernel with this packing
@@ -1785,14 +1796,8 @@ static int batch_configure(ldpc_batch* b, int pack, int threads, int ctas_per_sm
             if (rc) return fail(rc, "batch: code %zu does not fit pack %d: %s", i, pack, ldpc_last_error_string());
         }
         for (size_t i = 0; i < b->codes.size(); i++) b->pc_choice[i] = pack;
-        b->per_code = true;
         b->pack = pack;
-        b->kfn = nullptr;
-        b->grid = 0;
-        b->threads = 0;
-        b->smem = 0;
-        b->ctas_per_sm = 0;
-        b->key.clear();
+        batch_use_per_code(b);
         return LDPC_OK;
     }
     const int k = b->kind == LDPC_LEARNED ? 4 : b->kind;
@@ -1817,6 +1822,7 @@ static int batch_configure(ldpc_batch* b, int pack, int threads, int ctas_per_sm
             b->lv = lv;
             b->threads = threads;
             b->smem = (int)smem;
+            b->ctas_asked = ctas_per_sm;
             b->ctas_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, occ) : occ;
             b->grid = b->ctas_per_sm * b->sms;
             b->key.clear();
@@ -1843,6 +1849,7 @@ static int batch_configure(ldpc_batch* b, int pack, int threads, int ctas_per_sm
     b->lv = nullptr;
     b->threads = threads;
     b->smem = (int)smem;
+    b->ctas_asked = ctas_per_sm;
     b->ctas_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, occ) : occ;
     b->grid = b->ctas_per_sm * b->sms;
     b->key.clear();  // a captured graph no longer matches
@@ -1938,7 +1945,7 @@ extern "C" int ldpc_batch_set_learned(ldpc_batch* b, int n_iters, const int8_t* 
     if (b->per_code) {
         for (size_t i = 0; i < b->codes.size() && !rc; i++) rc = batch_code_decoder(b, (int)i, b->pc_choice[i], nullptr);
     } else {
-        rc = batch_configure(b, b->pack, b->threads, b->ctas_per_sm, false);
+        rc = batch_configure(b, b->pack, b->threads, b->ctas_asked, false);
     }
     if (rc) {
         b->off.clear();
@@ -1957,13 +1964,18 @@ extern "C" int ldpc_batch_set_early_stop(ldpc_batch* b, int enabled, int slack)
     if (!enabled && b->per_frame)
         return fail(LDPC_ERR_ARG, "the per-frame early stop of this batch cannot be turned off; create one without "
                                   "LDPC_FLAG_EARLY_STOP_FRAMES");
-    if (b->early != (enabled != 0)) batch_drop_decoders(b);  // per-code decoders: re-created with the flag
-    b->early = enabled != 0;
-    b->slack = (unsigned)slack;
-    if (b->lv) {  // the early stop is compiled into the byte kernel
-        int rc = batch_configure(b, b->pack, b->threads, b->ctas_per_sm, false);
-        if (rc) return rc;
+    if (b->early != (enabled != 0)) {
+        batch_drop_decoders(b);  // per-code decoders: re-created with the flag
+        b->early = enabled != 0;
+        if (b->lv) {  // the early stop is compiled into the byte kernel
+            int rc = batch_configure(b, b->pack, b->threads, b->ctas_asked, false);
+            if (rc) {
+                b->early = !b->early;
+                return rc;
+            }
+        }
     }
+    b->slack = (unsigned)slack;
     b->key.clear();
     return LDPC_OK;
 }
@@ -2080,15 +2092,6 @@ extern "C" int ldpc_batch_decode(ldpc_batch* b, const int8_t* const* d_llr, void
     }
     CUDA_TRY(cudaEventRecord(b->done, st));
     return LDPC_OK;
-}
-
-// the per-code strategy with the per-code choices as they stand
-static void batch_use_per_code(ldpc_batch* b)
-{
-    b->per_code = true;
-    b->kfn = nullptr;
-    b->grid = b->threads = b->smem = b->ctas_per_sm = 0;
-    b->key.clear();
 }
 
 // Per-code choice: for each code, every candidate kernel (BatchCand) is timed alone on that
