@@ -168,7 +168,6 @@ struct FrameStages {
     int slot_sz;              // bytes of a ring slot: the largest record plus its messages
     int* status;              // set to 1 when a wait on the copy engine gave up
     uint32_t c64 = 0x64646464u, c128 = 0x58005800u;  // lv::Regs
-    int stride;                 // two frames: rows of the largest stage, the lists' stride
     const unsigned char* none;  // two frames: the largest stage's message bytes, all 128 (no message)
 };
 
@@ -487,8 +486,9 @@ __global__ void __maxnreg__(80) decode_frame_kernel(const Plan P, const Job J,
 // beside the other frame (the lanes never mix, so that changes nothing the frame wrote).
 //
 // Stage record (Frame2Header): the rows' columns as lists of nv u16 in the layout of lv::Msg
-// (16-, 8-, 4- and 2-byte parts, so a row's columns and messages are a few wide accesses), then,
-// where the rows differ, a byte per row.  Its messages, in the ring slot behind the record, are
+// (16-, 8-, 4- and 2-byte parts, each an array over the stage's rows, so a row's columns and messages
+// are a few wide accesses, and every part is aligned for any number of rows), then, where the rows
+// differ, a byte per row.  Its messages, in the ring slot behind the record, are
 // lists of the same shape (the two frames' bytes 128 + m; in a pair's first iteration copies of
 // the byte 128).  A stage holds rows of one degree and class; a level of more than two kinds of rows
 // is one stage with lists of 4, 8 or 14 entries and a byte per row (mixed).  A thread stores its
@@ -509,9 +509,13 @@ __global__ void __maxnreg__(80) decode_frame_kernel(const Plan P, const Job J,
 // issues about 250 instructions (100 of them the fp16 arithmetic) at 0.54 per scheduler cycle with 3
 // row warps each.  IRA N = 64800 rate 1/2, 2048 frames, early stop (20 iterations on average), B200:
 // 15.7 ms before (messages stored back through the ring by bulk copies with a proxy fence in every
-// stage, edge by edge lists), 10.5 ms now; the 20000x10000 table, 1200 frames, 10 iterations 1.45 and
-// 0.99 ms.  Three rows a thread with 4 row warps instead of 12: 16.2 ms, two with 6 warps: 13.9 ms (too
-// few warps to issue from); the next stage's lists taken into registers before the barrier: 15.3 ms
+// stage, edge by edge lists), 10.2 to 10.4 ms now; the 20000x10000 table, 1200 frames, 10 iterations
+// 1.45 and 0.99 ms.  The lists are as long as their own stage: with the widest stage's length for all
+// of them, a kernel parameter, fixed iterations are 0.7 to 1.6 % faster (20000x10000, 600 frames: 596
+// and 605 us) and the early stop 2 % slower, but a serial code takes many times its edges (the
+// 64800x32400 table 547 MB of scratch and records, one wide level before 3000 rows of their own 2.5
+// GB).  Three rows a thread with 4 row warps instead of 12: 16.2 ms, two with 6 warps: 13.9 ms (too few
+// warps to issue from); the next stage's lists taken into registers before the barrier: 15.3 ms
 // (register moves around the dispatch).
 
 struct Frame2Header {
@@ -544,20 +548,20 @@ __device__ __forceinline__ void stage_load2(const FrameStages& S, const FrameSta
 // list length of a mixed stage of largest degree d
 __host__ __device__ constexpr int frame2_mixed(int d) { return d <= 4 ? 4 : (d <= 8 ? 8 : 14); }
 
-// Row t of a stage: d edges (MIXED: of lists of NV), lists `stride` rows apart; the new messages
-// go to the CTA's scratch gm at byte moff (a 32-bit offset: one add an access).
+// Row t of a stage of `rows` rows: d edges (MIXED: of lists of NV); the new messages go to the CTA's
+// scratch gm at byte moff (a 32-bit offset: one add an access).
 template <int KIND, int NV, bool MIXED>
 __device__ __forceinline__ void frame2_row(const lv::Regs& R, uint16_t* app, const char* cols, const char* msgs,
-                                           unsigned char* gm, uint32_t moff, int stride, int t, int d, bool noclip, uint32_t& odd, const uint16_t* lut)
+                                           unsigned char* gm, uint32_t moff, int rows, int t, int d, bool noclip, uint32_t& odd, const uint16_t* lut)
 {
     constexpr int W = lv::Msg<NV, 1>::W;
     uint32_t c[W], mw[W], B[1][NV], M[1][NV], o[1];
-    lv::Msg<NV, 1>::load(cols, stride, t, c);
+    lv::Msg<NV, 1>::load(cols, rows, t, c);
     auto var = [&](int j) { return (j & 1) ? c[j / 2] >> 16 : c[j / 2] & 0xffffu; };
     uint32_t w[NV];
 #pragma unroll
     for (int j = 0; j < NV; j++) w[j] = app[var(j)];
-    lv::Msg<NV, 1>::load(msgs, stride, t, mw);
+    lv::Msg<NV, 1>::load(msgs, rows, t, mw);
 #pragma unroll
     for (int j = 0; j < NV; j++) {
         B[0][j] = __byte_perm(w[j], R.c64, 0x4140);
@@ -574,15 +578,15 @@ __device__ __forceinline__ void frame2_row(const lv::Regs& R, uint16_t* app, con
     int k = 0;
     uint32_t p = moff;
 #pragma unroll
-    for (int b = 0; b + 16 <= 2 * NV; b += 16, k += 4, p += 16 * stride)
+    for (int b = 0; b + 16 <= 2 * NV; b += 16, k += 4, p += 16 * rows)
         *reinterpret_cast<uint4*>(gm + (p + 16u * t)) = make_uint4(mw[k], mw[k + 1], mw[k + 2], mw[k + 3]);
     if (NV & 4) {
         *reinterpret_cast<uint2*>(gm + (p + 8u * t)) = make_uint2(mw[k], mw[k + 1]);
-        p += 8 * stride, k += 2;
+        p += 8 * rows, k += 2;
     }
     if (NV & 2) {
         *reinterpret_cast<uint32_t*>(gm + (p + 4u * t)) = mw[k];
-        p += 4 * stride, k += 1;
+        p += 4 * rows, k += 1;
     }
     if (NV & 1) *reinterpret_cast<uint16_t*>(gm + (p + 2u * t)) = (uint16_t)mw[k];
 }
@@ -691,7 +695,7 @@ __global__ void __launch_bounds__(FRAME_MAX_THREADS + 32)
     __shared__ int s_abort;
     const bool producer = threadIdx.x == blockDim.x - 1;
     unsigned char* gmsg = S.msg + (long long)blockIdx.x * S.slot_bytes;
-    const int nst = S.nst, t = threadIdx.x, stride = S.stride;
+    const int nst = S.nst, t = threadIdx.x;
     const int group = nst >= 8 ? nst / 2 : 1;  // stages between two fences
     const lv::Regs R(S.c64, S.c128);
     if (threadIdx.x == 0) {
@@ -763,14 +767,14 @@ __global__ void __launch_bounds__(FRAME_MAX_THREADS + 32)
 #define LDPC_FRAME2_CASE(NV)                                                                                        \
     case NV: {                                                                                                      \
         const int cls = hd.z >> 8;                                                                                  \
-        frame2_row<KIND, NV, false>(R, app, cols, msgs, gmsg, hd.w, stride, t, NV, QUIRK && first && cls, odd,         \
+        frame2_row<KIND, NV, false>(R, app, cols, msgs, gmsg, hd.w, hd.x, t, NV, QUIRK && first && cls, odd,         \
                                     slut + 128 * cls);                                                              \
         break;                                                                                                      \
     }
 #define LDPC_FRAME2_MIXED(ID, NV)                                                                                  \
     case ID: {                                                                                                      \
-        const int b = *reinterpret_cast<const uint8_t*>(cols + ((2 * NV * stride + 15) & ~15) + t);                 \
-        frame2_row<KIND, NV, true>(R, app, cols, msgs, gmsg, hd.w, stride, t, b & 0x7f, QUIRK && first && b >> 7, odd,      \
+        const int b = *reinterpret_cast<const uint8_t*>(cols + ((2 * NV * hd.x + 15) & ~15) + t);                   \
+        frame2_row<KIND, NV, true>(R, app, cols, msgs, gmsg, hd.w, hd.x, t, b & 0x7f, QUIRK && first && b >> 7, odd,      \
                                    slut + 128 * (b >> 7));                                                          \
         break;                                                                                                      \
     }

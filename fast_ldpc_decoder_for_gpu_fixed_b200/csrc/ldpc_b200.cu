@@ -656,13 +656,11 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
             }
         }
     };
-    // two frames: rows [r0, r0 + rows) as lists of nv columns, `stride` rows apart; mixed: a byte
-    // per row
-    int stride = 8;
+    // two frames: rows [r0, r0 + rows) as lists of nv columns; mixed: a byte per row
     auto slot_bytes2 = [&](long long nv, int rows) { return hdr + 2 * pad16(2 * nv * rows) + pad16(rows); };
     auto emit2 = [&](int r0, int rows, int nv, bool mixed) {
         const int cls0 = c->row_class[c->order[r0]];
-        const long long list = pad16(2ll * nv * stride), rec_bytes = hdr + list + (mixed ? pad16(rows) : 0);
+        const long long list = pad16(2ll * nv * rows), rec_bytes = hdr + list + (mixed ? pad16(rows) : 0);
         unsigned char* b = add_stage(rec_bytes, list);
         *reinterpret_cast<Frame2Header*>(b) = {rows, (int)rec_bytes, mixed ? (nv == 4 ? 15 : (nv == 8 ? 16 : 17)) : nv | cls0 << 8,
                                              st.back().msg_off};
@@ -675,16 +673,16 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
                     if (base + part <= 2 * nv) base += part;
                     else part >>= 1;
                 }
-                *reinterpret_cast<uint16_t*>(b + hdr + (long long)base * stride + (long long)part * i + (2 * j - base)) =
+                *reinterpret_cast<uint16_t*>(b + hdr + (long long)base * rows + (long long)part * i + (2 * j - base)) =
                     (uint16_t)(j < dg ? c->cols[e0 + j] : 0);
             }
             if (mixed) b[hdr + list + i] = (unsigned char)(dg | c->row_class[r] << 7);
         }
     };
-    // two frames: the most rows of a stage, so that the longest lists at that stride fit a slot
-    const int nv_most = c->dmax <= 8 ? std::max(4, c->dmax) : 14;
+    // two frames: the most rows of a stage, so that the longest lists (those of a mixed stage) fit a slot
+    const int nv_most = frame2_mixed(c->dmax);
     int rows_cap = T;
-    while (two && rows_cap > 8 && slot_bytes2(nv_most, (rows_cap + 7) / 8 * 8) > slot_cap) rows_cap--;
+    while (two && rows_cap > 1 && slot_bytes2(nv_most, rows_cap) > slot_cap) rows_cap--;
     // two frames: calls f(first row, rows, list length, mixed) for the stages of a level
     auto level_stages = [&](const int2& lv, auto f) {
         const int end = lv.x + lv.y;
@@ -707,12 +705,6 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
             }
         }
     };
-    if (two) {
-        for (const int2& lv : c->levels)
-            level_stages(lv, [&](int, int rows, int, bool) { stride = std::max(stride, (rows + 7) / 8 * 8); });
-        if (slot_bytes2(nv_most, stride) > slot_cap)
-            return fail(LDPC_ERR_UNSUPPORTED, "LDPC_PACK_FRAME: no room for the stage ring next to two frames");
-    }
     for (const int2& lv : c->levels) {
         const int end = lv.x + lv.y;
         if (two) {
@@ -752,7 +744,6 @@ static int frame_stages_setup(ldpc_decoder* d, const ldpc_code* c, size_t base_s
     d->fst.st = d->d_fst;
     d->fst.rec = d->d_frec;
     d->fst.none = d->d_frec + rec_bytes;
-    d->fst.stride = stride;
     d->fst.slot_bytes = moff;
     d->fst.nst = (int)st.size();
     d->fst.slot_sz = slot_max;
