@@ -36,14 +36,20 @@
 // iterations before the last sigmoid - b of every variable (4 bytes) and S_f(t), in a
 // caller-provided stash.
 //
-// The row updates are unrolled for the code's row degrees, so that a row's values stay in
+// The row updates are unrolled for each row's own degree, so that a row's values stay in
 // registers: with loops over the degree they went through local memory, and the kernel waited
-// on that (1.44 G warp instructions at 0.44 per cycle).  sigmoid - b comes from the forward
+// on that (1.44 G warp instructions at 0.44 per cycle).  Unrolled for the largest degree of a class
+// (8, 16, 32) and predicated, a row also waits for the edges that it does not have: us of a forward
+// and backward pass, 600 frames, 5 iterations, with loops / by class / by degree: 1200x600 (degrees
+// 8 and 9) 4772 / 7164 / 3173; 816x408 (10) 1003 / 1085 / 570; 2048x384 (32) 987 / 1181 / 521;
+// 1944x972 (7 and 8) 384 / 209 / 170; 4000x2000 (6) 949 / 362 / 361.  Degrees above 16 spill beside 128
+// registers (476 bytes), which costs less than reading their columns twice (2048x384: 574).  sigmoid - b comes from the forward
 // pass's exp(-|z|) and is kept, so the backward pass evaluates no exponential.
 // N = 4096 QC code, 2048 frames, 10 iterations, every iteration weighted, forward and backward,
 // B200: 2.97 ms before, 1.15 ms now; its stash (0.67 GB) and sigmoids (0.30 GB), written and
 // read once, take 0.3 ms of that.
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "../../include/ldpc_b200.h"
@@ -152,8 +158,106 @@ __device__ __forceinline__ float frame_part(const TrainArgs& A, int n, long long
     return part;
 }
 
-// DT: the rows' degree (EXACT) or the most of it
-template <int DT, bool EXACT, bool VEC>
+// What the backward pass needs of a row's update: its minima, their edges and the signs.
+struct RowMinima {
+    float m1, m2;
+    int i1, i2;
+    uint32_t pos;
+};
+
+// The update of a row of D edges.  c: its first column in the code's table, the others m entries apart;
+// msg: its messages, likewise.
+template <int D>
+__device__ __forceinline__ RowMinima row_forward(const uint16_t* c, int m, float* a, float* msg, float al, float be, int quantized)
+{
+    RowMinima R{127.f, 127.f, 0, 1, 0u};
+    float tv[D];
+    int vo[D];
+#pragma unroll
+    for (int j = 0; j < D; j++) vo[j] = __ldg(c + j * m);
+#pragma unroll
+    for (int j = 0; j < D; j++) tv[j] = fminf(fmaxf(__fsub_rn(a[vo[j]], msg[j * m]), -128.f), 127.f);
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        const float ax = fminf(fabsf(tv[j]), 127.f);
+        R.pos |= (tv[j] > 0.f ? 1u : 0u) << j;
+        const bool lt1 = ax < R.m1, lt2 = ax < R.m2;
+        R.i2 = lt1 ? R.i1 : (lt2 ? j : R.i2);
+        R.i1 = lt1 ? j : R.i1;
+        R.m2 = fminf(R.m2, fmaxf(R.m1, ax));
+        R.m1 = fminf(R.m1, ax);
+    }
+    if (R.i2 == R.i1) R.i2 = R.i1 + 1 < D ? R.i1 + 1 : 0;  // all other magnitudes 127: any second edge
+    const float c1 = fminf(fmaxf(pre_mag(al, be, R.m2, quantized), 0.f), 31.f);
+    const float c2 = fminf(fmaxf(pre_mag(al, be, R.m1, quantized), 0.f), 31.f);
+    const uint32_t neg = (__popc(R.pos) & 1) ? R.pos : ~R.pos;  // bit j: the message of edge j is negative
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        const float mag = j == R.i1 ? c1 : c2;
+        const float mj = ((neg >> j) & 1) ? -mag : mag;
+        msg[j * m] = mj;
+        a[vo[j]] = fminf(fmaxf(__fadd_rn(tv[j], mj), -128.f), 127.f);
+    }
+    return R;
+}
+
+// The reverse of row_forward: a and msg hold the gradients of the APPs and of the messages after the row,
+// then those before it.  Adds the row's gradients of alpha and beta to da and db.
+template <int D>
+__device__ __forceinline__ void row_backward(const uint16_t* c, int m, float* a, float* msg, const RowMinima& R, float al, float be,
+                                             int quantized, float& da, float& db)
+{
+    const uint32_t neg = (__popc(R.pos) & 1) ? R.pos : ~R.pos;
+    float gt[D];
+    int vo[D];
+#pragma unroll
+    for (int j = 0; j < D; j++) vo[j] = __ldg(c + j * m);
+    float gc1 = 0.f, gc2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        gt[j] = a[vo[j]];                         // d/d a[v] after this row
+        const float gm = gt[j] + msg[j * m];      // d/d m_j: the APP and the next iteration
+        const float s = ((neg >> j) & 1) ? -gm : gm;
+        gc1 = j == R.i1 ? s : gc1;
+        gc2 += j == R.i1 ? 0.f : s;
+    }
+    float gm1 = 0.f, gm2 = 0.f;
+    const float y1 = pre_mag(al, be, R.m2, quantized), y2 = pre_mag(al, be, R.m1, quantized);
+    if (y1 > 0.f && y1 < 31.f) {
+        da += R.m2 * gc1;
+        db -= gc1;
+        gm2 = al * gc1;
+    }
+    if (y2 > 0.f && y2 < 31.f) {
+        da += R.m1 * gc2;
+        db -= gc2;
+        gm1 = al * gc2;
+    }
+    // min1 = |t_i1|, min2 = |t_i2|; d|t|/dt = +1 for t > 0, -1 otherwise
+    gm1 = ((R.pos >> R.i1) & 1) ? gm1 : -gm1;
+    gm2 = ((R.pos >> R.i2) & 1) ? gm2 : -gm2;
+#pragma unroll
+    for (int j = 0; j < D; j++) {
+        const float x = gt[j] + (j == R.i1 ? gm1 : (j == R.i2 ? gm2 : 0.f));
+        a[vo[j]] = x;     // d/d a[v] before this row
+        msg[j * m] = -x;  // d/d (this edge's message of iteration t-1)
+    }
+}
+
+// Calls f with the degree d (1 to MOST) as a compile-time constant.
+template <int MOST, int D = 1, class F>
+__device__ __forceinline__ void with_degree(int d, F f)
+{
+    if constexpr (D == MOST) {
+        f(std::integral_constant<int, D>());
+    } else {
+        if (d == D) f(std::integral_constant<int, D>());
+        else with_degree<MOST, D + 1>(d, f);
+    }
+}
+
+// DT: the largest degree; UNIFORM: every row has it
+template <int DT, bool UNIFORM, bool VEC>
 __global__ void __launch_bounds__(256, DT <= 8 ? 3 : 2) train_kernel(const Plan P, const TrainArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -182,48 +286,16 @@ __global__ void __launch_bounds__(256, DT <= 8 ? 3 : 2) train_kernel(const Plan 
         for (int l = 0; l < P.nlevels; l++) {
             const int2 lv = __ldg(P.levels + l);
             for (int r = lv.x + threadIdx.x; r < lv.x + lv.y; r += blockDim.x) {
-                const int d = EXACT ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
+                const int d = UNIFORM ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
                 const float al = g ? al1 : al0, be = g ? be1 : be0;
-                float tv[DT];
-                int vo[DT];
-#pragma unroll
-                for (int j = 0; j < DT; j++)
-                    if (EXACT || j < d) vo[j] = __ldg(P.cols + j * P.m + r);
-#pragma unroll
-                for (int j = 0; j < DT; j++)
-                    if (EXACT || j < d) tv[j] = fminf(fmaxf(__fsub_rn(a[vo[j]], msg[j * P.m + r]), -128.f), 127.f);
-                float m1 = 127.f, m2 = 127.f;
-                int i1 = 0, i2 = 1;
-                uint32_t pos = 0;
-#pragma unroll
-                for (int j = 0; j < DT; j++) {
-                    if (EXACT || j < d) {
-                        const float ax = fminf(fabsf(tv[j]), 127.f);
-                        pos |= (tv[j] > 0.f ? 1u : 0u) << j;
-                        const bool lt1 = ax < m1, lt2 = ax < m2;
-                        i2 = lt1 ? i1 : (lt2 ? j : i2);
-                        i1 = lt1 ? j : i1;
-                        m2 = fminf(m2, fmaxf(m1, ax));
-                        m1 = fminf(m1, ax);
-                    }
-                }
-                if (i2 == i1) i2 = i1 + 1 < d ? i1 + 1 : 0;  // all other magnitudes 127: any second edge
-                const uint32_t par = __popc(pos) & 1;
-                const float c1 = fminf(fmaxf(pre_mag(al, be, m2, A.quantized), 0.f), 31.f);
-                const float c2 = fminf(fmaxf(pre_mag(al, be, m1, A.quantized), 0.f), 31.f);
-                const uint32_t neg = par ? pos : ~pos;  // bit j: the message of edge j is negative
-#pragma unroll
-                for (int j = 0; j < DT; j++) {
-                    if (EXACT || j < d) {
-                        const float c = j == i1 ? c1 : c2;
-                        const float mj = ((neg >> j) & 1) ? -c : c;
-                        msg[j * P.m + r] = mj;
-                        a[vo[j]] = fminf(fmaxf(__fadd_rn(tv[j], mj), -128.f), 127.f);
-                    }
-                }
-                if (A.backward)
-                    A.stash[((size_t)f * T + t) * P.m + r] =
-                        make_uint4(__float_as_uint(m1), __float_as_uint(m2), (uint32_t)(i1 | (i2 << 8)), pos);
+                auto row = [&](auto D) {
+                    const RowMinima R = row_forward<D.value>(P.cols + r, P.m, a, msg + r, al, be, A.quantized);
+                    if (A.backward)
+                        A.stash[((size_t)f * T + t) * P.m + r] =
+                            make_uint4(__float_as_uint(R.m1), __float_as_uint(R.m2), (uint32_t)(R.i1 | (R.i2 << 8)), R.pos);
+                };
+                if constexpr (UNIFORM) row(std::integral_constant<int, DT>());
+                else with_degree<DT>(d, row);
             }
             __syncthreads();
         }
@@ -277,54 +349,18 @@ __global__ void __launch_bounds__(256, DT <= 8 ? 3 : 2) train_kernel(const Plan 
         for (int l = P.nlevels - 1; l >= 0; l--) {
             const int2 lv = __ldg(P.levels + l);
             for (int r = lv.x + threadIdx.x; r < lv.x + lv.y; r += blockDim.x) {
-                const int d = EXACT ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
+                const int d = UNIFORM ? DT : __ldg(P.rowdeg + r), g = __ldg(P.rowcls + r);
                 const uint4 st = A.stash[((size_t)f * T + t) * P.m + r];
                 const float al = g ? al1 : al0, be = g ? be1 : be0;
-                int vo[DT];
-#pragma unroll
-                for (int j = 0; j < DT; j++)
-                    if (EXACT || j < d) vo[j] = __ldg(P.cols + j * P.m + r);
-                const float m1 = __uint_as_float(st.x), m2 = __uint_as_float(st.y);
-                const int i1 = st.z & 0xff, i2 = (st.z >> 8) & 0xff;
-                const uint32_t pos = st.w, neg = (__popc(pos) & 1) ? pos : ~pos;
-                float gt[DT];
-                float gc1 = 0.f, gc2 = 0.f;
-#pragma unroll
-                for (int j = 0; j < DT; j++) {
-                    if (EXACT || j < d) {
-                        gt[j] = a[vo[j]];                             // d/d a[v] after this row
-                        const float gm = gt[j] + msg[j * P.m + r];    // d/d m_j: the APP and the next iteration
-                        const float s = ((neg >> j) & 1) ? -gm : gm;
-                        gc1 = j == i1 ? s : gc1;
-                        gc2 += j == i1 ? 0.f : s;
-                    }
-                }
-                float gm1 = 0.f, gm2 = 0.f;
-                const float y1 = pre_mag(al, be, m2, A.quantized), y2 = pre_mag(al, be, m1, A.quantized);
+                const RowMinima R{__uint_as_float(st.x), __uint_as_float(st.y), (int)(st.z & 0xff), (int)((st.z >> 8) & 0xff), st.w};
                 float da = 0.f, db = 0.f;
-                if (y1 > 0.f && y1 < 31.f) {
-                    da += m2 * gc1;
-                    db -= gc1;
-                    gm2 = al * gc1;
-                }
-                if (y2 > 0.f && y2 < 31.f) {
-                    da += m1 * gc2;
-                    db -= gc2;
-                    gm1 = al * gc2;
-                }
+                auto row = [&](auto D) {
+                    row_backward<D.value>(P.cols + r, P.m, a, msg + r, R, al, be, A.quantized, da, db);
+                };
+                if constexpr (UNIFORM) row(std::integral_constant<int, DT>());
+                else with_degree<DT>(d, row);
                 ga0 += g ? 0.f : da, gb0 += g ? 0.f : db;
                 ga1 += g ? da : 0.f, gb1 += g ? db : 0.f;
-                // min1 = |t_i1|, min2 = |t_i2|; d|t|/dt = +1 for t > 0, -1 otherwise
-                gm1 = ((pos >> i1) & 1) ? gm1 : -gm1;
-                gm2 = ((pos >> i2) & 1) ? gm2 : -gm2;
-#pragma unroll
-                for (int j = 0; j < DT; j++) {
-                    if (EXACT || j < d) {
-                        const float x = gt[j] + (j == i1 ? gm1 : (j == i2 ? gm2 : 0.f));
-                        a[vo[j]] = x;              // d/d a[v] before this row
-                        msg[j * P.m + r] = -x;     // d/d (this edge's message of iteration t-1)
-                    }
-                }
             }
             __syncthreads();
         }
