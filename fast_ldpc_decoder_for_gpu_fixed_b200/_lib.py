@@ -41,6 +41,7 @@ SIGNATURES = {
     "ldpc_decode_device": (_I, [_P, _P, _P, _SZ, _I, _I, _P, _P, _P]),
     "ldpc_decode_device_state": (_I, [_P, _P, _P, _SZ, _I, _P, _P, _P, _P]),
     "ldpc_decoder_info": (_I, [_P, _P]),
+    "ldpc_decoder_level_info": (_I, [_P, _P]),
     "ldpc_decoder_set_learned": (_I, [_P, _I, _P, _P]),
     "ldpc_decoder_set_early_stop": (_I, [_P, _I, _I]),
     "ldpc_decoder_status": (_I, [_P, _P]),

@@ -119,6 +119,8 @@ struct ldpc_decoder {
     int path = 0;
     // paths 0 and 2 on decode_level_bytes_kernel: its schedule (level_setup)
     bool bytes = false;
+    int level_fp = 0;         // frame pairs per thread
+    bool level_half = false;  // one frame pair per CTA
     LevelPlan lplan{};
     unsigned char* d_level = nullptr;
     bool pf_levels = false;  // path 0 with the per-frame early stop (SIMD4; counts per frame)
@@ -775,6 +777,8 @@ static int level_select(ldpc_decoder* d, const ldpc_code* c, int kind, bool half
     d->pf_levels = per_frame;
     d->path = half ? 2 : 0;
     d->bytes = true;
+    d->level_fp = lc.fp;
+    d->level_half = lc.half;
     d->smem = (int)smem;
     d->threads = lc.threads;
     return LDPC_OK;
@@ -1132,6 +1136,16 @@ extern "C" int ldpc_decoder_info(const ldpc_decoder* d, int* info)
     info[5] = d->ctas_per_sm;
     info[6] = d->regs;
     info[7] = d->path;
+    return LDPC_OK;
+}
+
+extern "C" int ldpc_decoder_level_info(const ldpc_decoder* d, int* info)
+{
+    if (!d || !info) return fail(LDPC_ERR_ARG, "ldpc_decoder_level_info: null pointer");
+    info[0] = d->bytes;
+    info[1] = d->level_fp;
+    info[2] = d->level_half;
+    info[3] = d->bytes ? d->lplan.nstep : 0;
     return LDPC_OK;
 }
 

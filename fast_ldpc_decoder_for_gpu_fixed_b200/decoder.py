@@ -112,6 +112,12 @@ class Decoder:
         keys = ("kind", "pack", "nb_frames", "threads", "smem", "ctas_per_sm", "regs", "path")
         return dict(zip(keys, list(a)))
 
+    def level_info(self):
+        """The level kernel's choice for this decoder (ldpc_decoder_level_info)."""
+        a = (ctypes.c_int * 4)()
+        _lib.check(_lib.lib().ldpc_decoder_level_info(self.handle, a))
+        return dict(zip(("bytes", "pairs_per_thread", "pair_per_cta", "steps"), list(a)))
+
     def set_early_stop(self, enabled=True, slack=_lib.EARLY_STOP_DEFAULT_SLACK):
         """Syndrome early stop on/off and its slack (ldpc_decoder_set_early_stop)."""
         _lib.check(_lib.lib().ldpc_decoder_set_early_stop(self.handle, int(bool(enabled)), int(slack)))

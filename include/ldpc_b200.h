@@ -330,6 +330,12 @@ int ldpc_decoder_set_early_stop(ldpc_decoder* dec, int enabled, int slack);
  * LDPC_PACK_F16X2_SPLIT) */
 int ldpc_decoder_info(const ldpc_decoder* dec, int* info);
 
+/* info[0..3] of a level-scheduled decoder (paths 0 and 2): 1 = the byte-storage level kernel, 0 =
+ * another kernel (info[1..3] are 0 then); frame pairs a thread updates at once (2 or 1); 1 = one
+ * frame pair per CTA; steps of an iteration.  For tests and diagnosis: the choice follows the code
+ * and nb_frames and gives the same decisions either way. */
+int ldpc_decoder_level_info(const ldpc_decoder* dec, int* info);
+
 int ldpc_decoder_destroy(ldpc_decoder* dec);
 
 /* Kernel status of a decoder (no reference counterpart): *status = 1 when a kernel of
