@@ -118,6 +118,20 @@ __device__ __forceinline__ void qc_row_parity(const QcCheck& C, int l, int k, in
     }
 }
 
+// KIND_LEARNED: the (k, k) and (b, b) words of every iteration into shared memory (the head of each
+// [iteration][row group] table, see ldpc_decoder_set_learned; QC rows are of group 0), so that no
+// iteration waits on a global load and a barrier for its constants.  All threads; a barrier before the
+// first use.  A CTA may have fewer threads than there are iterations.
+template <int KIND>
+__device__ __forceinline__ void qc_load_constants(const Job& J, uint2* s_kb)
+{
+    for (int t = threadIdx.x; t < J.lut_its; t += blockDim.x) {
+        uint2 kb = *reinterpret_cast<const uint2*>(J.lut + t * 256);
+        if (KIND == KIND_LEARNED_OFS) kb.y = h2::add(kb.y, 0x37803780u);  // b + 15/32 = -offset (scale 1)
+        s_kb[t] = kb;
+    }
+}
+
 // true when row k of some layer in [L0, L1) has odd hard-decision parity in one of
 // the CTA's frames (see the early stop in decode_qc_kernel)
 template <int DT, bool EXACT, int L0, int L1, bool POW2, int WPT>
@@ -209,17 +223,10 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
     QcCheck chk{};
     if (ET) chk = qc_check_setup<DT, EXACT, (ET ? L : 0)>(Q, s_chk, smem_raw);
     __shared__ unsigned s_odd[2];
-    // KIND_LEARNED: the (k, k) and (b, b) words of every iteration and row group, loaded
-    // once (the head of each [iteration][group] table, see ldpc_decoder_set_learned), so
-    // that no iteration waits on a global load and a barrier for its constants
     constexpr bool LRN = KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS;
-    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1][2];
+    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1];
     if (k < 2) s_odd[k] = 0;
-    if (LRN && k < 2 * J.lut_its) {
-        uint2 kb = *reinterpret_cast<const uint2*>(J.lut + (k >> 1) * 256 + (k & 1) * 128);
-        if (KIND == KIND_LEARNED_OFS) kb.y = h2::add(kb.y, 0x37803780u);  // b + 15/32 = -offset (scale 1)
-        s_kb[k >> 1][k & 1] = kb;
-    }
+    if (LRN) qc_load_constants<KIND>(J, s_kb);
     // the odd-row count of the early stop: a +-1 accumulator on the FMA pipe (row(), CMODE 2);
     // 2NMS keeps the exact popcount, which its own rule tests against zero
     constexpr int CM = ((ET == 1 || ET == 2) && KIND != KIND_2NMS) ? 2 : 0;
@@ -288,7 +295,7 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
             }
             uint32_t lk = 0, lb = 0;  // LEARNED constants of this layer's class (registers only within the layer)
             if (KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS) {
-                const uint2 kb = s_kb[lt][0];
+                const uint2 kb = s_kb[lt];
                 lk = kb.x;
                 lb = kb.y;
             }
@@ -456,12 +463,9 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
     const QcCheck chk = qc_check_setup<DT, false, L>(Q, s_chk, smem_raw);
     __shared__ unsigned s_odd[2];
     constexpr bool LRN = KIND == KIND_LEARNED;
-    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1][2];
+    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1];
     if (threadIdx.x < 2) s_odd[threadIdx.x] = 0;
-    if (LRN && threadIdx.x < 2 * J.lut_its) {
-        const int t = threadIdx.x;
-        s_kb[t >> 1][t & 1] = *reinterpret_cast<const uint2*>(J.lut + (t >> 1) * 256 + (t & 1) * 128);
-    }
+    if (LRN) qc_load_constants<KIND>(J, s_kb);
     constexpr int CM = ET ? 2 : 0;
 
     Plan P;
@@ -497,7 +501,7 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][0];
+                const uint2 kb = s_kb[lt];
                 lk = kb.x;
                 lb = kb.y;
             }
@@ -656,7 +660,7 @@ __device__ __forceinline__ unsigned cta_or_pairs(unsigned bits)
 // decisions are codewords (live = 0) or J.iters.  Every thread of the CTA calls it.
 template <int KIND, int DT, bool EXACT, int L, bool POW2>
 __device__ __forceinline__ void qc_one_pair(const QCParams& Q, const Job& J, char* appb, const QcCheck& chk, int hoff,
-                                            uint32_t (&m)[L][DT], const uint2 (*s_kb)[2], int& it, unsigned& live)
+                                            uint32_t (&m)[L][DT], const uint2* s_kb, int& it, unsigned& live)
 {
     constexpr bool LRN = KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS;
     constexpr int LS = L > 3 ? 2 : 1;
@@ -681,7 +685,7 @@ __device__ __forceinline__ void qc_one_pair(const QCParams& Q, const Job& J, cha
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][0];
+                const uint2 kb = s_kb[lt];
                 lk = kb.x;
                 lb = kb.y;
             }
@@ -732,12 +736,8 @@ __global__ void __launch_bounds__(256, 2) decode_qc_pairs_kernel(const __grid_co
     __shared__ __align__(16) int2 s_chk[L * DT];
     const QcCheck chk = qc_check_setup<DT, EXACT, L>(Q, s_chk, smem_raw);
     constexpr bool LRN = KIND == KIND_LEARNED || KIND == KIND_LEARNED_OFS;
-    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1][2];
-    if (LRN && k < 2 * J.lut_its) {
-        uint2 kb = *reinterpret_cast<const uint2*>(J.lut + (k >> 1) * 256 + (k & 1) * 128);
-        if (KIND == KIND_LEARNED_OFS) kb.y = h2::add(kb.y, 0x37803780u);  // b + 15/32 = -offset (scale 1)
-        s_kb[k >> 1][k & 1] = kb;
-    }
+    __shared__ uint2 s_kb[LRN ? QC_LUT_ITS : 1];
+    if (LRN) qc_load_constants<KIND>(J, s_kb);
     // the successor word's LLRs into L2, as in decode_qc_kernel
     if (threadIdx.x == 0 && !J.gen && !J.interleaved && (Q.n & 3) == 0) {
         unsigned nsm;
@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(256, 2) decode_qc_pairs_kernel(const __grid_co
             }
             uint32_t lk = 0, lb = 0;
             if (LRN) {
-                const uint2 kb = s_kb[lt][0];
+                const uint2 kb = s_kb[lt];
                 lk = kb.x;
                 lb = kb.y;
             }
@@ -888,16 +888,15 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
     __shared__ long long s_slot[QC_STAGE];  // frame staged in each slot, -1 = none (the frames run out)
     __shared__ int s_src[4];           // refill: the slot each done lane takes
     __shared__ int s_head;             // the slot holding the earliest staged frame
-    __shared__ __align__(16) uint32_t s_kb[2][4];  // LEARNED, per row group: k words of pair-words 0, 1, then b words
-    __shared__ uint16_t s_tab[QC_LUT_ITS][2][2];  // LEARNED: fp16 (k, b) per iteration and row group
+    __shared__ __align__(16) uint32_t s_kb[4];  // LEARNED: k words of pair-words 0, 1, then b words
+    __shared__ uint16_t s_tab[QC_LUT_ITS][2];   // LEARNED: fp16 (k, b) per iteration
 
     if (k < 2) {
         s_cnt[0][k] = s_cnt[1][k] = 0;
         s_bad[0][k] = s_bad[1][k] = 0;
     }
     if (KIND == KIND_LEARNED)
-        for (int i = k; i < 4 * J.lut_its; i += blockDim.x)
-            s_tab[i >> 2][(i >> 1) & 1][i & 1] = J.lut[(i >> 2) * 256 + ((i >> 1) & 1) * 128 + 2 * (i & 1)];
+        for (int i = k; i < 2 * J.lut_its; i += blockDim.x) s_tab[i >> 1][i & 1] = J.lut[(i >> 1) * 256 + 2 * (i & 1)];
     if (k == 0) {
         // this CTA's frames: blockIdx.x + G j; lanes take j = 0..3, the slots j = 4..7
         for (int i = 0; i < 4; i++) {
@@ -946,11 +945,8 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
             uint16_t* h = reinterpret_cast<uint16_t*>(s_kb);
             if (KIND == KIND_LEARNED) {
                 const int t = it < J.lut_its ? it : J.lut_its - 1;
-#pragma unroll
-                for (int g = 0; g < 2; g++) {
-                    h[8 * g + k] = s_tab[t][g][0];
-                    h[8 * g + 4 + k] = s_tab[t][g][1];
-                }
+                h[k] = s_tab[t][0];
+                h[4 + k] = s_tab[t][1];
             }
         }
         __syncthreads();
@@ -974,7 +970,7 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
             }
             uint32_t lk0 = 0, lk1 = 0, lb0 = 0, lb1 = 0;
             if (KIND == KIND_LEARNED) {
-                const uint4 q = reinterpret_cast<const uint4*>(s_kb)[0];
+                const uint4 q = *reinterpret_cast<const uint4*>(s_kb);
                 lk0 = q.x;
                 lk1 = q.y;
                 lb0 = q.z;
