@@ -201,11 +201,11 @@ __device__ __forceinline__ void count_group_errors(const Plan& P, const Job& J, 
             e[k] += bit != ref;
         }
     }
+    // a QC kernel's last warp may have fewer than 32 threads
+    const int lanes = (int)blockDim.x - (int)(threadIdx.x & ~31u);
+    const unsigned wmask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) e[k] += __shfl_xor_sync(0xffffffffu, e[k], o);
-    }
+    for (int k = 0; k < 4; k++) e[k] = __reduce_add_sync(wmask, e[k]);
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int k = 0; k < 4; k++) part[k][threadIdx.x >> 5] = e[k];
