@@ -82,7 +82,10 @@ __device__ __forceinline__ void write_frame(const Plan& P, const Job& J, long lo
     const int n = P.n;
     const long long lf = f - 4 * J.word0;
     if (J.counts) {
-        __shared__ int part[FRAME_MAX_THREADS / 32 + 1];
+        // by the frame's parity: the two frames of a CTA may follow each other without a barrier, and
+        // thread 0 still sums the first one's parts
+        __shared__ int parts[2][FRAME_MAX_THREADS / 32 + 1];
+        int* part = parts[f & 1];
         int e = 0;
         const uint8_t* cw = J.cw ? J.cw + ((unsigned long long)f % (unsigned long long)J.n_cw) * n : nullptr;
         for (int v = threadIdx.x; v < J.n_vars; v += blockDim.x) e += (x(v) > 0) != (cw ? cw[v] != 0 : false);

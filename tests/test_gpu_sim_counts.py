@@ -1,9 +1,10 @@
 """The error counts of ldpc_simulate against its own decisions, where the counting can go wrong: CTAs whose
-last warp is not full (QC kernels with a lifting size that is no multiple of 32)."""
+last warp is not full (QC kernels with a lifting size that is no multiple of 32), and the two frames of a
+long-code CTA, which are counted one right after the other."""
 import numpy as np
 import pytest
 
-from fast_ldpc_decoder_for_gpu_fixed_b200 import Decoder
+from fast_ldpc_decoder_for_gpu_fixed_b200 import Decoder, load_table
 from fast_ldpc_decoder_for_gpu_fixed_b200.codes import qc_irregular, qc_regular
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +34,12 @@ def test_last_warp_not_full(cuda, base, z, pack, n_vars):
     path, got, want = _counts(code, 40, 2, 1.1, n_vars, pack=pack)
     assert path == (1 if base == "regular" else {"F16X2": 4, "F16X2_SPLIT": 7, "SIMD4": 0}[pack])
     assert got == want and want[1] > 0
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("n_vars", [0, 1, 33, 576])
+@pytest.mark.parametrize("name", ["576x288", "1944x972"])
+def test_two_frames_of_a_cta(cuda, name, n_vars, early):
+    path, got, want = _counts(load_table(name), 300, 3, 0.9, n_vars, pack="FRAME", early_stop=early)
+    assert path == 3
+    assert got == want
