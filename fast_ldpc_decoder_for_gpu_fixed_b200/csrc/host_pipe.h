@@ -12,6 +12,7 @@
 // A call takes a pipe for its time (HostPipes): pinned memory takes milliseconds to allocate, so at
 // most two idle pipes are kept for later calls, of any decoder, until no decoder is left.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -30,18 +31,18 @@
 namespace ldpc {
 
 // Threads that share a loop with the caller.  Asleep between calls; from wake() to rest() they spin on
-// the loop counter, since a wake-up through the kernel takes as long as a piece's copy, but for at most
-// SPIN without a new loop: then they sleep until there is one (the caller waits for the GPU, and other
-// calls and processes need the cores).  16 cores, one caller, us a call and us of CPU time, spinning
-// throughout / 30 / 100 / 300 us: 4000x2000, 4096 frames, 20 iterations 950, 5570 / 960, 5180 / 950,
-// 5540 / 985, 5780; with 200 iterations 7060, 42 200 / 7110, 11 900 / 7110, 14 800 / 7080, 22 200;
-// 280 frames, 10 iterations 172, 950 / 182, 550 / 178, 880 / 186, 1020; 20000x10000, 1200 frames, 50
-// iterations 7210, 43 000 / 7560, 14 200 / 7430, 14 400 / 7530, 17 000 (its waits are the longest: the
-// helpers are woken for each piece).  Six callers at once, 4000x2000, 4096 frames: 1120, 15 700 / 950,
-// 9430 / 1070, 10 200 / 1020, 11 000.
+// the loop counter, since a wake-up through the kernel takes as long as a piece's copy, but once CALL has
+// passed since wake() only for SPIN without a new loop: then they sleep until there is one (the caller
+// waits for the GPU, and other calls and processes need the cores).  16 cores, one caller, us a call and
+// us of CPU time, spinning throughout / so: 4000x2000, 280 frames, 10 iterations 173, 950 / 171, 945; 4096
+// frames, 20 iterations 930 to 950, 5440 to 5570 / 930, 5440; 200 iterations 7060, 42 200 / 7095, 14 800;
+// 20000x10000, 1200 frames, 50 iterations, whose waits are the longest, 7240, 43 200 / 7350, 14 700.  With
+// SPIN alone from the start of a call the short ones take 2 to 4 % longer (280 frames 178), with 30 us of
+// it 182, with 300 us the long ones 22 200 us of CPU time.  Six callers at once, 4000x2000, 4096 frames:
+// 1070 to 1630, 15 000 to 20 000 / 1050, 10 000.
 class HostTeam {
 public:
-    static constexpr std::chrono::microseconds SPIN{100};
+    static constexpr std::chrono::microseconds SPIN{100}, CALL{500};
     explicit HostTeam(int helpers)
     {
         try {
@@ -93,16 +94,19 @@ private:
     {
         unsigned seen = 0, woken = 0;
         for (;;) {
+            bool called;
             {
                 std::unique_lock<std::mutex> l(m_);
                 asleep_.fetch_add(1);
                 cv_.wait(l, [&] { return stop_ || wakes_ != woken || turn_.load() != seen; });
                 asleep_.fetch_sub(1);
                 if (stop_) return;
+                called = wakes_ != woken;  // by wake(), not by a loop
                 woken = wakes_;
             }
             // rest() comes after each() has returned: no turn is left undone
             auto last = std::chrono::steady_clock::now();
+            if (called) last += CALL - SPIN;
             while (awake_.load(std::memory_order_acquire)) {
                 const unsigned t = turn_.load(std::memory_order_acquire);
                 if (t == seen) {
@@ -113,7 +117,7 @@ private:
                 seen = t;
                 (*f_)(part, size());
                 done_.fetch_add(1, std::memory_order_release);
-                last = std::chrono::steady_clock::now();
+                last = std::max(last, std::chrono::steady_clock::now());
             }
         }
     }
