@@ -185,8 +185,9 @@ __device__ __forceinline__ void read_group(const Plan& P, const Job& J, long lon
 
 // Error counting of the group's 4 frames against the transmitted codewords
 // (ber_analyzer/CErrorAnalyzer.cpp:142-158): bits among the first n_vars whose
-// decision (x > 0) differs from the codeword bit.  Every thread of the CTA calls it.
-template <class F>
+// decision (x > 0) differs from the codeword bit.  Every thread of the CTA calls it.  FULL: every warp
+// has 32 threads (the QC kernels' last one may have fewer).
+template <bool FULL = true, class F>
 __device__ __forceinline__ void count_group_errors(const Plan& P, const Job& J, long long g, F get, int kmask)
 {
     __shared__ int part[4][32];
@@ -201,11 +202,17 @@ __device__ __forceinline__ void count_group_errors(const Plan& P, const Job& J, 
             e[k] += bit != ref;
         }
     }
-    // a QC kernel's last warp may have fewer than 32 threads
     const int lanes = (int)blockDim.x - (int)(threadIdx.x & ~31u);
     const unsigned wmask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
 #pragma unroll
-    for (int k = 0; k < 4; k++) e[k] = __reduce_add_sync(wmask, e[k]);
+    for (int k = 0; k < 4; k++) {
+        if (!FULL) {
+            e[k] = __reduce_add_sync(wmask, e[k]);
+            continue;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) e[k] += __shfl_xor_sync(0xffffffffu, e[k], o);
+    }
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int k = 0; k < 4; k++) part[k][threadIdx.x >> 5] = e[k];
@@ -226,13 +233,13 @@ __device__ __forceinline__ void count_group_errors(const Plan& P, const Job& J, 
     }
 }
 
-// Writes hard decisions; get(v) returns the 4-frame byte word (values as x) of variable v.
-template <class F>
+// Writes hard decisions; get(v) returns the 4-frame byte word (values as x) of variable v.  FULL: as above.
+template <bool FULL = true, class F>
 __device__ __forceinline__ void write_group(const Plan& P, const Job& J, long long g, F get, int kmask = 0xF)
 {
     const int n = P.n;
     const long long lg = g - J.word0;
-    if (J.counts) count_group_errors(P, J, g, get, kmask);
+    if (J.counts) count_group_errors<FULL>(P, J, g, get, kmask);
     if (!J.out) return;
     if (!J.out_packed) {
         uint8_t* o = reinterpret_cast<uint8_t*>(J.out) + 4 * lg * n;

@@ -82,15 +82,15 @@ __device__ __forceinline__ void write_frame(const Plan& P, const Job& J, long lo
     const int n = P.n;
     const long long lf = f - 4 * J.word0;
     if (J.counts) {
-        // by the frame's parity: the two frames of a CTA may follow each other without a barrier, and
-        // thread 0 still sums the first one's parts
-        __shared__ int parts[2][FRAME_MAX_THREADS / 32 + 1];
-        int* part = parts[f & 1];
+        __shared__ int part[FRAME_MAX_THREADS / 32 + 1];
         int e = 0;
         const uint8_t* cw = J.cw ? J.cw + ((unsigned long long)f % (unsigned long long)J.n_cw) * n : nullptr;
         for (int v = threadIdx.x; v < J.n_vars; v += blockDim.x) e += (x(v) > 0) != (cw ? cw[v] != 0 : false);
 #pragma unroll
         for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        // the two frames of a CTA may follow each other without a barrier: thread 0 may still sum the
+        // first one's parts (separate parts for the two cost the kernel 1.5 %, by its registers)
+        __syncthreads();
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
         __syncthreads();
         if (threadIdx.x == 0) {

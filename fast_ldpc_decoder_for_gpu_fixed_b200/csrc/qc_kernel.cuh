@@ -22,7 +22,10 @@
 // by masks and a no-clip branch that no QC code takes (all its rows are of class 0); 2.14 ms
 // without.  The deployed decoder (early stop per frame pair): 1.57 and 1.54 ms, and 1.51 ms with
 // the checks' (shift, block) pairs in a shared-memory table (their generic loads from the parameters
-// took a tenth of the kernel's instructions).
+// took a tenth of the kernel's instructions).  Where no word stops (1.0 dB) the exact-gate kernels take
+// 2.36 ms per pair and 2.33 per word against 2.14 with fixed iterations: 10.5 and 9 % an iteration (4.4 %
+// before the row update got cheaper, which gave the fixed kernel 9 % and the pairs kernel, at 128
+// registers with 8 bytes spilled, 3 %).
 #pragma once
 #include "decode_kernel.cuh"
 
@@ -388,7 +391,7 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
     if (WPT == 1) {
         // frames 2h, 2h+1 only; the word's iteration count is the larger of its two pairs
         // (the host zeroes d_iters_out before the launch)
-        write_group(P, J, g, [&](int v) { return AccessHalf::get(app1, v, h); }, 3 << (2 * h));
+        write_group<false>(P, J, g, [&](int v) { return AccessHalf::get(app1, v, h); }, 3 << (2 * h));
         if (J.iters_out && threadIdx.x == 0) atomicMax(J.iters_out + (g - J.word0), executed);
         if (J.synd_out) {
             const unsigned bad = passed ? 0u
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(256, WPT == 2 ? 2 : 1) decode_qc_kernel(const 
         }
         return;
     }
-    write_group(P, J, g, [&](int v) { uint2 a = app[v]; return Access<PackF16x2>::unbias(a.x, a.y); });
+    write_group<false>(P, J, g, [&](int v) { uint2 a = app[v]; return Access<PackF16x2>::unbias(a.x, a.y); });
     if (J.iters_out && threadIdx.x == 0) J.iters_out[g - J.word0] = executed;
     if (J.synd_out) {
         const unsigned bad = passed ? 0u
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(512) decode_qc_split_kernel(const __grid_const
     }
     // frames 2h, 2h+1 only; the word's iteration count is the larger of its two pairs
     // (the host zeroes d_iters_out before the launch)
-    write_group(P, J, g, [&](int v) { return AccessHalf::get(app1, v, h); }, 3 << (2 * h));
+    write_group<false>(P, J, g, [&](int v) { return AccessHalf::get(app1, v, h); }, 3 << (2 * h));
     if (J.iters_out && threadIdx.x == 0) atomicMax(J.iters_out + (g - J.word0), executed);
     if (J.synd_out) {
         const unsigned bad = passed || !lead ? 0u : qc_rows_unsat_mask<DT, false, 0, L, false, 1>(chk, k);
@@ -832,7 +835,7 @@ __global__ void __launch_bounds__(256, 2) decode_qc_pairs_kernel(const __grid_co
     else if (live == 2u)
         qc_one_pair<KIND, DT, EXACT, L, POW2>(Q, J, appb, chk, 4, msg[1], s_kb, it, live);
 
-    write_group(P, J, g, [&](int v) { uint2 a = app[v]; return Access<PackF16x2>::unbias(a.x, a.y); });
+    write_group<false>(P, J, g, [&](int v) { uint2 a = app[v]; return Access<PackF16x2>::unbias(a.x, a.y); });
     if (J.iters_out && threadIdx.x == 0) J.iters_out[g - J.word0] = it;
     if (J.synd_out) {
         // a stopped pair holds codewords; the rest are checked on their final APP
