@@ -8,9 +8,10 @@
 // thread and 3 or 4 CTAs of 128 threads fitted a multiprocessor; with 96 registers 5 do.  us
 // before and after: the above 6890 / 6256; the same codes, 300 words 278 / 259; each frame
 // stopping on its own, 20 000 words 4782 / 3451; 20 fixed iterations, 20 000 words 4130 / 3959.
-// With 72 registers the row update spills.  Without the early stop the schedule's pointers are
-// better kept in registers (3959; from shared memory 4152), with it in shared memory (6256; in
-// registers 6357).
+// The row update spills at 96 registers: 44 to 60 bytes without the early stop, 72 to 80 with it, 116 to
+// 124 with the stop per frame (148 to 280 with 72 registers).  Without the early stop the schedule's
+// pointers are better kept in registers (3959; from shared memory 4152), with it in shared memory
+// (6256; in registers 6357).
 #include "batch_kernel.cuh"
 
 namespace ldpc {

@@ -74,7 +74,7 @@ const void* kernel_table_batch_pf(int kind, int variant)
 
 size_t batch_code_bytes() { return sizeof(BatchCode); }
 
-// fills one BatchCode record on the host (the struct stays private to this file)
+// fills one BatchCode record on the host (the caller knows its size alone)
 void batch_code_fill(void* rec, const Plan& plan, const LevelPlan& lplan, const int8_t* llr, void* out, int32_t* iters_out, uint8_t* synd_out,
                      long long words, long long first_item, int quirk, int out_packed, int variant)
 {

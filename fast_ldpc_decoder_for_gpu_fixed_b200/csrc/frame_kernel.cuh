@@ -512,10 +512,10 @@ __global__ void __maxnreg__(80) decode_frame_kernel(const Plan P, const Job J,
 // issues about 250 instructions (100 of them the fp16 arithmetic) at 0.54 per scheduler cycle with 3
 // row warps each.  IRA N = 64800 rate 1/2, 2048 frames, early stop (20 iterations on average), B200:
 // 15.7 ms before (messages stored back through the ring by bulk copies with a proxy fence in every
-// stage, edge by edge lists), 10.2 to 10.4 ms now; the 20000x10000 table, 1200 frames, 10 iterations
+// stage, edge by edge lists), 10.2 to 10.5 ms now; the 20000x10000 table, 1200 frames, 10 iterations
 // 1.45 and 0.99 ms.  The lists are as long as their own stage: with the widest stage's length for all
-// of them, a kernel parameter, fixed iterations are 0.7 to 1.6 % faster (20000x10000, 600 frames: 596
-// and 605 us) and the early stop 2 % slower, but a serial code takes many times its edges (the
+// of them, a kernel parameter, fixed iterations are 0.7 to 1.6 % faster (20000x10000, 600 frames: 594
+// and 604 us) and the early stop 2 to 4 % slower, but a serial code takes many times its edges (the
 // 64800x32400 table 547 MB of scratch and records, one wide level before 3000 rows of their own 2.5
 // GB).  Three rows a thread with 4 row warps instead of 12: 16.2 ms, two with 6 warps: 13.9 ms (too few
 // warps to issue from); the next stage's lists taken into registers before the barrier: 15.3 ms

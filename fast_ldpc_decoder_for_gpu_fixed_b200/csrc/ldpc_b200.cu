@@ -1292,7 +1292,13 @@ static int host_decode_status(ldpc_decoder* d)
 
 // Whether the staged host decode takes the call: both buffers pageable, at least a megabyte of
 // LLRs in the frame-major layout (xMS reads all of its interleaved input at once), a frame's packed
-// decisions within a piece.
+// decisions within a piece.  us a call, direct / staged, 20 iterations (8000x4000: 10), 16 cores:
+//   pageable: 4000x2000 0.24 MB 202 / 182, 0.98 MB 301 / 217, 3.9 MB 674 / 380, 15.6 MB 2640 / 903;
+//     576x288 0.28 MB 135 / 117, 8.8 MB 2270 / 632; 8000x4000 30.5 MB 4250 / 1660
+//   pinned: 4000x2000 0.24 MB 173 / 182, 0.98 MB 204 to 258 / 217, 3.9 MB 560 to 690 / 380, 15.6 MB
+//     978 / 908; 8000x4000 30.5 MB 1337 / 1720
+// So a megabyte is on the safe side for pageable buffers, and pinned ones, which keep the direct copies,
+// would gain between about 1 and 16 MB (a byte a decision over PCIe) and lose outside.
 static bool host_pipe_serves(const ldpc_decoder* d, const void* in, const void* out, size_t in_bytes)
 {
     if (d->kind == LDPC_XMS || in_bytes < (1 << 20) || ((size_t)d->n + 7) / 8 > HostPipe::OUT_BYTES) return false;

@@ -212,7 +212,10 @@ inline void level_records(const Rows& H, const LevelSteps& order, LevelSchedule&
 // words: two pairs, steps of 96 lanes and 128 threads 624, 96 threads 653, 128 lanes 645, 64
 // lanes 627, one pair 674; 1944x972, 777 words: 96 threads (6 words a multiprocessor, one round)
 // 478, 128 threads (5) 520; 576x288, one word: one pair 68, two pairs 88; 2304x1152, 1024 words:
-// 96 lanes 229, 192 lanes 236, one word: 42 and 40.
+// 96 lanes 229, 192 lanes 236, one word: 42 and 40.  The registers a thread (72, 96) are those of the
+// two-pair kernels without the early stop; with it they take up to 122 (per frame), so there the rule
+// counts more words as resident than are, and its cost is the lower bound of it.
+// Host time to choose and lay out a schedule: 0.1 ms for 576x288, 0.7 for 4000x2000, 2.2 for 9972x4986.
 // lds: shared memory beside the messages; fixed_threads: the CTA width, 0 = free; may_half: one
 // frame pair per CTA is allowed (it pays while the words leave multiprocessors idle).  False when
 // the code has no such schedule.

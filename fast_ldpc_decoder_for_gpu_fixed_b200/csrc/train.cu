@@ -47,7 +47,9 @@
 // pass's exp(-|z|) and is kept, so the backward pass evaluates no exponential.
 // N = 4096 QC code, 2048 frames, 10 iterations, every iteration weighted, forward and backward,
 // B200: 2.97 ms before, 1.15 ms now; its stash (0.67 GB) and sigmoids (0.30 GB), written and
-// read once, take 0.3 ms of that.
+// read once, take 0.3 ms of that.  What bounds it (592 frames, counters): issue slots 58 % and the ALU pipe 57 %
+// busy with 4.8 warps a scheduler (registers and shared memory both allow 3 CTAs of 8 warps), DRAM 13 %;
+// the rest is latency, of the columns' and the stash's loads first, with too few warps to hide it.
 #include <cstdint>
 #include <type_traits>
 #include <cuda_runtime.h>

@@ -192,7 +192,9 @@ void ldpc_code_destroy(ldpc_code* code);
  * nb_frames >= 1 is accepted.  The decoder owns its device buffers; the code
  * may be destroyed after this call.  pack = LDPC_PACK_*; flags = 0 or
  * LDPC_FLAG_EARLY_STOP, LDPC_FLAG_EARLY_STOP_FRAMES, LDPC_FLAG_EARLY_STOP_PAIRS,
- * LDPC_FLAG_FLOODING. */
+ * LDPC_FLAG_FLOODING.  Creating one allocates device memory and lays out the code's rows: 1.2 to
+ * 1.8 ms for codes of up to 4000 variables, 3.2 ms for 9972x4986 (of it 0.1 to 2.2 ms of host time for
+ * the byte-storage level kernel's schedule); the kernel's shape is chosen for nb_frames. */
 int ldpc_decoder_create(ldpc_decoder** out, const ldpc_code* code, int kind, size_t nb_frames,
                         int pack, int flags);
 
@@ -322,9 +324,9 @@ int ldpc_decoder_set_early_stop(ldpc_decoder* dec, int enabled, int slack);
  * per CTA, CTAs per SM, registers per thread, kernel path (0 = level
  * scheduled, 1 = QC register-message, 2 = level scheduled, fixed iterations:
  * LDPC_PACK_F16X2 for every kind but 2NMS (4 frames per CTA in byte storage, 2 where the words
- * leave multiprocessors idle, and 2 in fp16 for the codes and kinds byte storage does not serve), 3 = one frame per CTA with
- * packed row state: LDPC_PACK_FRAME, 4 = QC register-message with 2 frames per
- * CTA, see LDPC_PACK_F16X2, 5 = QC register-message with per-frame early stop,
+ * leave multiprocessors idle, and 2 in fp16 for the codes and kinds byte storage does not
+ * serve), 3 = long codes, messages off chip: LDPC_PACK_FRAME (two frames per CTA where they fit,
+ * else one), 4 = QC register-message with 2 frames per CTA, see LDPC_PACK_F16X2, 5 = QC register-message with per-frame early stop,
  * see LDPC_FLAG_EARLY_STOP_FRAMES, 6 = level kernel with the flooding schedule, see
  * LDPC_FLAG_FLOODING, 7 = QC register-message with 2 frames per CTA and split rows, see
  * LDPC_PACK_F16X2_SPLIT) */
