@@ -203,15 +203,15 @@ __device__ __forceinline__ void count_group_errors(const Plan& P, const Job& J, 
         }
     }
     const int lanes = (int)blockDim.x - (int)(threadIdx.x & ~31u);
-    const unsigned wmask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
+    [[maybe_unused]] const unsigned wmask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        if (!FULL) {
-            e[k] = __reduce_add_sync(wmask, e[k]);
-            continue;
-        }
+        if constexpr (FULL) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) e[k] += __shfl_xor_sync(0xffffffffu, e[k], o);
+            for (int o = 16; o; o >>= 1) e[k] += __shfl_xor_sync(0xffffffffu, e[k], o);
+        } else {
+            e[k] = __reduce_add_sync(wmask, e[k]);
+        }
     }
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
