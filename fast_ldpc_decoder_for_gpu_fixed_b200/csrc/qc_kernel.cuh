@@ -588,12 +588,20 @@ __device__ __forceinline__ void qc_put_lane(const int8_t* src, uint16_t* apph, i
     }
 }
 
+// word-interleaved input: byte f % 4 of word v * words + f / 4
+__device__ __forceinline__ const int8_t* qc_interleaved(const Job& J, long long f, int v)
+{
+    return J.llr + 4 * (v * J.total_words + (f >> 2)) + (f & 3);
+}
+
 // starts the copy of frame f's LLRs into a staging slot: cp.async (16-byte pieces,
 // completed by cp.async.wait_all) when source and size allow it, else plain copies
 __device__ __forceinline__ void qc_stage_frame(const Job& J, int8_t* slot, int n, long long f, bool async16)
 {
     const int8_t* src = J.llr + f * n;
-    if (async16) {
+    if (J.interleaved) {
+        for (int v = threadIdx.x; v < n; v += blockDim.x) slot[v] = __ldg(qc_interleaved(J, f, v));
+    } else if (async16) {
         const unsigned dst = (unsigned)__cvta_generic_to_shared(slot);
         for (int c = threadIdx.x; c < (n >> 4); c += blockDim.x)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * c), "l"(src + 16 * c) : "memory");
@@ -884,7 +892,7 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
     const long long G = gridDim.x;
     __shared__ __align__(16) int2 s_chk[L * DT];
     const QcCheck check = qc_check_setup<DT, EXACT, L>(Q, s_chk, smem_raw);
-    const bool async16 = ((reinterpret_cast<uintptr_t>(J.llr) | (uintptr_t)Q.n) & 15) == 0;
+    const bool async16 = !J.interleaved && ((reinterpret_cast<uintptr_t>(J.llr) | (uintptr_t)Q.n) & 15) == 0;
     __shared__ unsigned s_cnt[2][2];   // odd rows per lane (16-bit fields of pair-words 0, 1), by iteration parity
     __shared__ unsigned s_bad[2][2];   // unsatisfied lanes of the two check stages, by iteration parity
     __shared__ long long s_frame[4];   // frame of each lane, -1 = idle
@@ -923,7 +931,13 @@ __global__ void __launch_bounds__(256, 2) decode_qc_refill_kernel(const __grid_c
         const long long f = s_frame[i];
         if (f >= 0) {
             act |= 1u << i;
-            qc_put_lane<true>(J.llr + f * Q.n, apph, Q.n, i);
+            if (J.interleaved)
+                for (int v = k; v < Q.n; v += blockDim.x) {
+                    const uint32_t y = (uint32_t)(uint8_t)__ldg(qc_interleaved(J, f, v)) ^ 0x7fu;
+                    apph[4 * v + i] = (uint16_t)h2::add(__byte_perm(y, 0x6464u, 0x4140), h2::CNEG1024);
+                }
+            else
+                qc_put_lane<true>(J.llr + f * Q.n, apph, Q.n, i);
         }
     }
     if (!act) {
