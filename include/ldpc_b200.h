@@ -192,8 +192,8 @@ void ldpc_code_destroy(ldpc_code* code);
  * nb_frames >= 1 is accepted.  The decoder owns its device buffers; the code
  * may be destroyed after this call.  pack = LDPC_PACK_*; flags = 0 or
  * LDPC_FLAG_EARLY_STOP, LDPC_FLAG_EARLY_STOP_FRAMES, LDPC_FLAG_EARLY_STOP_PAIRS,
- * LDPC_FLAG_FLOODING.  Creating one allocates device memory and lays out the code's rows: 1.2 to
- * 1.8 ms for codes of up to 4000 variables, 3.2 ms for 9972x4986 (of it 0.1 to 2.2 ms of host time for
+ * LDPC_FLAG_FLOODING.  Creating one allocates device memory and lays out the code's rows: 0.7 to
+ * 1.9 ms for codes of up to 4000 variables, 3.2 ms for 9972x4986 (of it 0.1 to 2.2 ms of host time for
  * the byte-storage level kernel's schedule); the kernel's shape is chosen for nb_frames. */
 int ldpc_decoder_create(ldpc_decoder** out, const ldpc_code* code, int kind, size_t nb_frames,
                         int pack, int flags);
