@@ -34,15 +34,15 @@ namespace ldpc {
 // the loop counter, since a wake-up through the kernel takes as long as a piece's copy, but once CALL has
 // passed since wake() only for SPIN without a new loop: then they sleep until there is one (the caller
 // waits for the GPU, and other calls and processes need the cores).  16 cores, one caller, us a call and
-// us of CPU time, spinning throughout / so: 4000x2000, 280 frames, 10 iterations 173, 950 / 171, 945; 4096
-// frames, 20 iterations 930 to 950, 5440 to 5570 / 930, 5440; 200 iterations 7060, 42 200 / 7095, 14 800;
-// 20000x10000, 1200 frames, 50 iterations, whose waits are the longest, 7240, 43 200 / 7350, 14 700.  With
-// SPIN alone from the start of a call the short ones take 2 to 4 % longer (280 frames 178), with 30 us of
-// it 182, with 300 us the long ones 22 200 us of CPU time.  Six callers at once, 4000x2000, 4096 frames:
-// 1070 to 1630, 15 000 to 20 000 / 1050, 10 000.
+// us of CPU time, spinning throughout / so: 4000x2000, 280 frames, 10 iterations 173, 950 / 172, 950; 4096
+// frames, 20 iterations 930 to 950, 5440 to 5570 / 940, 5500; 200 iterations 7060, 42 200 / 7100, 20 200;
+// 20000x10000, 1200 frames, 50 iterations, whose waits are the longest, 7240, 43 200 / 7390, 15 800.  With
+// a SPIN of 100 us the 200 iterations take 14 800 us of CPU time, but one call in ten of 0.91 ms takes 0.12
+// ms longer (a helper asleep when the last piece comes); without CALL calls of 0.2 ms take 2 to 4 % longer.
+// Six callers at once, 4000x2000, 4096 frames: 1070 to 1630, 15 000 to 20 000 / 940, 10 600.
 class HostTeam {
 public:
-    static constexpr std::chrono::microseconds SPIN{100}, CALL{500};
+    static constexpr std::chrono::microseconds SPIN{250}, CALL{500};
     explicit HostTeam(int helpers)
     {
         try {
